@@ -4,7 +4,7 @@
 //   3 x { k_rhs_ext + k_rhs_comp (face fluxes, cell-centric over each cell's
 //         extended / compact entries),
 //         k_rk_prim (rk3Step fused with the primitive/packed-state update),
-//         k_grad (compact-CSR velocity gradient) }
+//         k_grad (velocity gradient over the compact stencil) }
 //   k_step_end (Vreman SGS, material properties, Gibbs sensor, calcCfl ->
 //               next dt, NaN flag; once per step)
 // Face sums are taken per cell over that cell's own face list in a fixed
@@ -84,21 +84,6 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return fma(r, e, r);
 }
 
-// Sum / max over the G lanes of a group (xor butterfly: every lane ends with
-// the same, order-fixed result).  All 32 lanes of the warp must call it.
-template <int G>
-__device__ __forceinline__ double group_sum(double v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-template <int G>
-__device__ __forceinline__ double group_max(double v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // 256-bit read-only global loads (sm_100): a 32 B-aligned record piece per
 // lane in one instruction, one sector per lane.
 __device__ __forceinline__ double4 ld4(const void* p) {
@@ -111,32 +96,26 @@ __device__ __forceinline__ void st4(void* p, double a, double b, double c, doubl
 }
 
 
-// dudx of one cell
-__device__ __forceinline__ void load_Vg(const VRec* base, int j, double g[9]) {
+// dudx of one cell (g[8] with the last sector: symh, symp, mu_lam)
+__device__ __forceinline__ double4 load_Vg(const VRec* base, int j, double g[9]) {
   const double* p = reinterpret_cast<const double*>(base + j);
-  const double2 b = __ldg(reinterpret_cast<const double2*>(p + 6));
-  const double4 c = ld4(p + 8), d = ld4(p + 12);
-  g[0] = b.x; g[1] = b.y;
-  g[2] = c.x; g[3] = c.y; g[4] = c.z; g[5] = c.w;
-  g[6] = d.x; g[7] = d.y; g[8] = d.z;
+  const double4 b = ld4(p + 4), c = ld4(p + 8), d = ld4(p + 12);
+  g[0] = b.x; g[1] = b.y; g[2] = b.z; g[3] = b.w;
+  g[4] = c.x; g[5] = c.y; g[6] = c.z; g[7] = c.w;
+  g[8] = d.x;
+  return d;
 }
 
 // ---- shared-memory staging of neighbour records -------------------------
-// Record arrays in shared memory hold records of R 16-byte chunks (R = 2, 4
-// or 8).  Chunk c of record j sits at 16-byte slot (j mod P)*R + (c xor
-// ((j/P) mod R)) of 128-byte row j/P, P = 8/R records per row: the same chunk
-// of records j..j+7 lands in eight different 16-byte bank groups, so the G
-// lanes of a cell reading different neighbours rarely conflict.
-template <int R>
-__device__ __forceinline__ int swz(int j, int c) {
-  constexpr int P = 8 / R;
-  return (j / P) * 8 + (j % P) * R + (c ^ ((j / P) % R));
-}
-// 16-byte chunks a record array of n records occupies (whole rows)
-template <int R>
-__host__ __device__ constexpr int swz_chunks(int n) {
-  return ((n * R + 7) / 8) * 8;
-}
+// A record array in shared memory holds its records' 16-byte chunks plane by
+// plane: chunk c of record j at 16-byte slot c * pl + j, with a plane length pl
+// that is the same for the whole launch (so that a chunk's address is a
+// register plus a uniform offset).  The same chunk of records that differ
+// modulo 8 lies in different bank groups, which is what the order of the
+// entries within their rows is chosen for.  pl is 8 / R modulo 8 (R chunks per
+// record): the chunks of consecutive records that eight lanes write while
+// staging fall into different bank groups too.
+__host__ __device__ constexpr int plane_len(int n, int R) { return (n + 7) / 8 * 8 + (R >= 8 ? 1 : R >= 4 ? 2 : R >= 2 ? 4 : 0); }
 
 __device__ __forceinline__ void cp_async16(int4* dst, const void* src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -152,79 +131,75 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(unsigned(e - a)) : "memory");
 }
 
-// L2 prefetch of the per-entry streams (six planes of TB-byte values and a
-// 16-bit index) of entries [k0, k1); threads 0..6 of the CTA issue one each.
-template <class TB>
-__device__ __forceinline__ void prefetch_entries(const TB* planes, long long stride,
-                                                 const unsigned short* idx, long long k0, long long k1) {
-  const int t = threadIdx.x;
-  if (t < 6)
-    prefetch_l2(planes + t * stride + k0, (k1 - k0) * static_cast<long long>(sizeof(TB)));
-  else if (t == 6)
-    prefetch_l2(idx + k0, (k1 - k0) * 2);
-}
+// ---- row streams ---------------------------------------------------------
+// A warp walks the rows of one slice, one of `parts` warps taking rows part,
+// part + parts, ...  A lane's values of a row are stored in C chunks of type T
+// (16, 8 or 4 bytes), chunk c of the 32 lanes side by side, so that a warp loads
+// whole lines and an entry takes few load instructions.  The rows are used
+// once and come from DRAM: kAhead of its rows ahead the warp asks for the row
+// (ROWB bytes) to be brought into L2, and the slice's index stream is asked for
+// when the slice begins, before the item's records are staged.  What is left
+// of an L2 hit's latency is covered by the SM's other warps.
+constexpr int kAhead = 3;
+constexpr int kIdxBatch = 8;  // local indices a lane of the once-per-step kernel loads at a time
+template <int ROWB, class T, int C>
+struct Rows {
+  const T* src;               // the lane's first chunk of its next row
+  const unsigned short* idx;  // the lane's local index in that row
+  int left;                   // the lane's rows still to come
+  int jn;                     // the local index of the next row
 
-// The entries a staged kernel reads in round `sub` of item `it` (cells
-// it.cell0 + [sub*cpr, (sub+1)*cpr)): extended (COMP false) or compact.
-template <bool COMP, class TB>
-__device__ __forceinline__ void prefetch_round(const MeshDev& m, const TB* planes, const Item& it, int sub,
-                                               int cpr) {
-  const int a = min(sub * cpr, it.ncell), b = min((sub + 1) * cpr, it.ncell);
-  if (a >= b || threadIdx.x >= 7) return;
-  const long long* o = COMP ? m.qoff : m.off;
-  prefetch_entries(planes, COMP ? m.Q : m.E, COMP ? m.clidx : m.lidx, __ldg(o + it.cell0 + a),
-                   __ldg(o + it.cell0 + b));
-}
-
-// The streams the once-per-step kernel reads in round `sub` of item `it`:
-// the extended entries' local indices, the compact entries' local indices,
-// unit normals and areas.
-__device__ __forceinline__ void prefetch_end(const MeshDev& m, const Item& it, int sub, int cpr) {
-  const int a = min(sub * cpr, it.ncell), b = min((sub + 1) * cpr, it.ncell);
-  const int t = threadIdx.x;
-  if (a >= b || t >= 6) return;
-  if (t == 0) {
-    const long long k0 = __ldg(m.off + it.cell0 + a), k1 = __ldg(m.off + it.cell0 + b);
-    prefetch_l2(m.lidx + k0, (k1 - k0) * 2);
-    return;
+  __device__ __forceinline__ void start(const void* base, const unsigned short* lists, size_t row0, int rows, int n,
+                                        int part, int parts) {
+    const int lane = int(threadIdx.x) & 31;
+    left = max(0, (n - part + parts - 1) / parts);
+    src = reinterpret_cast<const T*>(static_cast<const char*>(base) + (row0 + part) * ROWB) + lane;
+    idx = lists + (row0 + part) * kSlice + lane;
+    if (lane < kAhead) {
+      if (part + lane * parts < rows)
+        prefetch_l2(static_cast<const char*>(base) + (row0 + part + lane * parts) * ROWB, ROWB);
+    } else if (lane == kAhead && part == 0) {
+      prefetch_l2(lists + row0 * kSlice, (long long)rows * kSlice * 2);
+    }
+    jn = (left > 0) ? __ldg(idx) : 0;
   }
-  const long long q0 = __ldg(m.qoff + it.cell0 + a), q1 = __ldg(m.qoff + it.cell0 + b);
-  if (t == 5)
-    prefetch_l2(m.clidx + q0, (q1 - q0) * 2);
-  else
-    prefetch_l2(m.qg + (t - 1) * m.Q + q0, (q1 - q0) * 8);
-}
-
-// the gradient kernel's streams: local indices and three coefficient planes
-// (TB-byte values) of the round's gradient entries
-template <class TB>
-__device__ __forceinline__ void prefetch_grad(const MeshDev& m, const TB* gx, const TB* gy, const TB* gz,
-                                              const Item& it, int sub, int cpr) {
-  const int a = min(sub * cpr, it.ncell), b = min((sub + 1) * cpr, it.ncell);
-  const int t = threadIdx.x;
-  if (a >= b || t >= 4) return;
-  const long long k0 = __ldg(m.coff + it.cell0 + a), k1 = __ldg(m.coff + it.cell0 + b);
-  if (t == 0) {
-    prefetch_l2(m.cglidx + k0, (k1 - k0) * 2);
-    return;
+  // the lane's chunks of its next row and the local index of its neighbour
+  __device__ __forceinline__ int next(int parts, T (&v)[C]) {
+    if ((threadIdx.x & 31) == 0 && left > kAhead)
+      prefetch_l2(reinterpret_cast<const char*>(src) + size_t(kAhead * parts) * ROWB, ROWB);
+#pragma unroll
+    for (int c = 0; c < C; ++c) v[c] = __ldg(src + 32 * c);
+    const int j = jn;
+    src = reinterpret_cast<const T*>(reinterpret_cast<const char*>(src) + size_t(parts) * ROWB);
+    idx += kSlice * parts;
+    if (--left > 0) jn = __ldg(idx);
+    return j;
   }
-  const TB* p = (t == 1) ? gx : (t == 2) ? gy : gz;
-  prefetch_l2(p + k0, (k1 - k0) * static_cast<long long>(sizeof(TB)));
-}
+};
 
-// Copy the records (R chunks each) of an item's cells, then of its halo
-// cells, into a swizzled shared array.  Asynchronous: complete with
-// stage_wait().
-// RS: the global record's size in chunks (the first R are copied).
-template <int R, int RS = R>
-__device__ __forceinline__ void stage_records(int4* sm, const void* base, const Item& it,
+// Copy the first R chunks of the records (RS chunks each) of an item's cells,
+// then of its halo cells, into planes of length pl.  Asynchronous: complete
+// with stage_wait().  Each thread reads its next kStage halo indices before it
+// copies the first of their chunks: with one index at a time the chain of
+// index and copy latencies took 0.11 of 1.72 ms of k_rhs_ext at 128^3.
+constexpr int kStage = 4;
+template <int R, int RS>
+__device__ __forceinline__ void stage_records(int4* sm, int pl, const void* base, const Item& it,
                                               const int* __restrict__ halo, int nh) {
   const int4* b = reinterpret_cast<const int4*>(base);
-  const int nu = it.ncell + nh;
-  for (int x = threadIdx.x; x < nu * R; x += blockDim.x) {
-    const int u = x / R, c = x % R;
-    const int cell = (u < it.ncell) ? it.cell0 + u : __ldg(halo + (u - it.ncell));
-    cp_async16(sm + swz<R>(u, c), b + size_t(cell) * RS + c);
+  const int nx = (it.ncell + nh) * R, T = blockDim.x;
+  for (int x0 = threadIdx.x; x0 < nx; x0 += kStage * T) {
+    int cell[kStage];
+#pragma unroll
+    for (int k = 0; k < kStage; ++k) {
+      const int u = (x0 + k * T) / R;
+      cell[k] = (u < it.ncell) ? it.cell0 + u : (x0 + k * T < nx) ? __ldg(halo + (u - it.ncell)) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kStage; ++k) {
+      const int x = x0 + k * T, u = x / R, c = x % R;
+      if (x < nx) cp_async16(sm + c * pl + u, b + size_t(cell[k]) * RS + c);
+    }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -233,155 +208,159 @@ __device__ __forceinline__ void stage_wait() {
   __syncthreads();
 }
 
-__device__ __forceinline__ void smem_L(const int4* sm, int j, LRec& r) {
-  const double2* p = reinterpret_cast<const double2*>(sm);
-  const double2 a = p[swz<4>(j, 0)], b = p[swz<4>(j, 1)], c = p[swz<4>(j, 2)], d = p[swz<4>(j, 3)];
+// what the extended faces' flux reads of a cell; h = K p v, K = gamma/(gamma-1)
+struct ERec {
+  double u[3], v, p, rho;
+};
+constexpr int kEChunks = 3;  // the first 48 B of an LRec
+__device__ __forceinline__ void smem_E(const int4* sm, int pl, int j, ERec& r) {
+  const double2* p = reinterpret_cast<const double2*>(sm) + j;
+  const double2 a = p[0], b = p[pl], c = p[2 * pl];
+  r.u[0] = a.x; r.u[1] = a.y; r.u[2] = b.x; r.v = b.y;
+  r.p = c.x; r.rho = c.y;
+}
+__device__ __forceinline__ void smem_L(const int4* sm, int pl, int j, LRec& r) {
+  const double2* p = reinterpret_cast<const double2*>(sm) + j;
+  const double2 a = p[0], b = p[pl], c = p[2 * pl], d = p[3 * pl];
   r.u[0] = a.x; r.u[1] = a.y; r.u[2] = b.x; r.sp_vol = b.y;
-  r.p = c.x; r.h = c.y; r.rho = d.x; r.sos = d.y;
+  r.p = c.x; r.rho = c.y; r.h = d.x; r.sos = d.y;
 }
 
-
 // field-wise sum of two cells' viscous records in shared memory
-__device__ __forceinline__ void smem_V_sum(const int4* sm, int a, int b, VRec& r) {
-  const double2* p = reinterpret_cast<const double2*>(sm);
-  double2 x = p[swz<8>(a, 0)], y = p[swz<8>(b, 0)];
+__device__ __forceinline__ void smem_V_sum(const int4* sm, int pl, int a, int b, VRec& r) {
+  const double2* p = reinterpret_cast<const double2*>(sm) + a;
+  const double2* q = reinterpret_cast<const double2*>(sm) + b;
+  double2 x = p[0], y = q[0];
   r.mu_total = x.x + y.x; r.loc_total = x.y + y.y;
-  x = p[swz<8>(a, 1)]; y = p[swz<8>(b, 1)];
+  x = p[pl]; y = q[pl];
   r.a_sgs = x.x + y.x; r.fgr = x.y + y.y;
-  x = p[swz<8>(a, 2)]; y = p[swz<8>(b, 2)];
-  r.symh = x.x + y.x; r.symp = x.y + y.y;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    x = p[swz<8>(a, 3 + c)];
-    y = p[swz<8>(b, 3 + c)];
+    x = p[(2 + c) * pl];
+    y = q[(2 + c) * pl];
     r.g[2 * c] = x.x + y.x;
     r.g[2 * c + 1] = x.y + y.y;
   }
-  r.g[8] = p[swz<8>(a, 7)].x + p[swz<8>(b, 7)].x;
+  x = p[6 * pl]; y = q[6 * pl];
+  r.g[8] = x.x + y.x; r.symh = x.y + y.y;
+  r.symp = p[7 * pl].x + q[7 * pl].x;
 }
 
-__device__ __forceinline__ double4 smem_Q(const int4* sm, int j) {
-  const double2* p = reinterpret_cast<const double2*>(sm);
-  const double2 a = p[swz<2>(j, 0)], b = p[swz<2>(j, 1)];
+__device__ __forceinline__ double4 smem_Q(const int4* sm, int pl, int j) {
+  const double2* p = reinterpret_cast<const double2*>(sm) + j;
+  const double2 a = p[0], b = p[pl];
   return make_double4(a.x, a.y, b.x, b.y);
 }
 
-struct Flux {
-  double rho, ru[3], rE;
-};
-
 // Skew-symmetric flux plus its symmetric "c" part (IdealGasSolverFlux.hpp:
-// 9-39 and 41-90) of the face a -> b, as one 5-vector.  The reference's two
-// functions produce the same terms; here they are grouped around the total
-// mass flux M = mdot + dmdot:
+// 9-39 and 41-90) of the face a -> b, subtracted from the five sums and
+// returned as its mass flux.  The reference's two functions produce the same
+// terms; here they are grouped around the total mass flux M = mdot + dmdot:
 //   F.rho = M
 //   F.ru  = p_f n + dp c + M uf + mdot_c du
 //   F.rE  = M h_f + mdot_c (dh + uf.du)
-// (mdot = rho_f uf.n, dmdot = uf.c drho + rho_f du.c, mdot_c = rho_f uf.c).
+// (mdot = rho_f uf.n, dmdot = uf.c drho + rho_f du.c, mdot_c = rho_f uf.c), on
+// the sums s = u_a + u_b = 2 uf and r = rho_f / 2, whose halves are exact.
 // Every term changes sign exactly under (a <-> b, n -> -n, c kept), so the
 // two cells of a face see exactly opposite fluxes.
-__device__ __forceinline__ void ext_flux(double F[5], const double n[3], const double c[3], const LRec& a,
-                                         const LRec& b) {
-  const double rho_f = 2.0 * rcp_nr(a.sp_vol + b.sp_vol);
+__device__ __forceinline__ double ext_flux_sub(double acc[5], const double n[3], const double c[3], const ERec& a,
+                                               double ha, const ERec& b, double K) {
+  const double r = rcp_nr(a.v + b.v);
+  double s[3], du[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    s[d] = a.u[d] + b.u[d];
+    du[d] = b.u[d] - a.u[d];
+  }
+  const double sn = s[0] * n[0] + s[1] * n[1] + s[2] * n[2];
+  const double sc = s[0] * c[0] + s[1] * c[1] + s[2] * c[2];
+  const double duc = du[0] * c[0] + du[1] * c[1] + du[2] * c[2];
+  const double uaub = a.u[0] * b.u[0] + a.u[1] * b.u[1] + a.u[2] * b.u[2];
+  const double sdu = s[0] * du[0] + s[1] * du[1] + s[2] * du[2];
+  const double mdot_c = sc * r;
+  const double M = sn * r + (0.5 * (sc * (b.rho - a.rho)) + 2.0 * (r * duc));
+  const double hb = K * (b.p * b.v);
+  const double hp = 0.5 * (a.p + b.p), dp = b.p - a.p, hM = 0.5 * M;
+  const double dH = (hb - ha) + 0.5 * sdu;
+  acc[0] -= M;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    acc[1 + d] -= hp * n[d];
+    acc[1 + d] -= dp * c[d];
+    acc[1 + d] -= hM * s[d];
+    acc[1 + d] -= mdot_c * du[d];
+  }
+  acc[4] -= hM * ((ha + hb) + uaub);
+  acc[4] -= mdot_c * dH;
+  return M;
+}
+
+// Compact closures (IdealGasSolverFlux.hpp:93-215) of the face a -> b, taken
+// from the five sums' negatives, i.e. acc += their value; returns the mass
+// flux they take from the face's.  The closures use the two cells' properties
+// and gradients only through their sums: vs holds V_a + V_b field by field.
+// With uf = (u_a + u_b)/2 and du = u_b - u_a the reference's differences of
+// squares are products: (|u_b|^2 - |u_a|^2)/2 = uf.du and (un_b^2 - un_a^2)/2 =
+// un_m dun.
+__device__ __forceinline__ double compact_flux_add(double acc[5], const double un_[3], double area, double aod,
+                                                   double delta, const LRec& a, const LRec& b, const VRec& vs) {
+  const double half_aod = 0.5 * aod;
+  const double mu_area = 0.5 * vs.mu_total * area;
+  const double mu_aod = vs.mu_total * half_aod;
+  const double k_aod = vs.loc_total * half_aod;
   double uf[3], du[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     uf[d] = 0.5 * (a.u[d] + b.u[d]);
     du[d] = b.u[d] - a.u[d];
   }
-  const double un = uf[0] * n[0] + uf[1] * n[1] + uf[2] * n[2];
-  const double uc = uf[0] * c[0] + uf[1] * c[1] + uf[2] * c[2];
-  const double duc = du[0] * c[0] + du[1] * c[1] + du[2] * c[2];
-  const double uaub = a.u[0] * b.u[0] + a.u[1] * b.u[1] + a.u[2] * b.u[2];
+  const double un_m = uf[0] * un_[0] + uf[1] * un_[1] + uf[2] * un_[2];
+  const double dun = du[0] * un_[0] + du[1] * un_[1] + du[2] * un_[2];
   const double ufdu = uf[0] * du[0] + uf[1] * du[1] + uf[2] * du[2];
-  const double mdot = un * rho_f;
-  const double dmdot = uc * (b.rho - a.rho) + rho_f * duc;
-  const double mdot_c = uc * rho_f;
-  const double M = mdot + dmdot;
-  const double p_f = 0.5 * (a.p + b.p);
-  const double dp = b.p - a.p;
+  const double uaub = a.u[0] * b.u[0] + a.u[1] * b.u[1] + a.u[2] * b.u[2];
   const double h_f = 0.5 * ((a.h + b.h) + uaub);
-  const double dH = (b.h - a.h) + ufdu;
-  F[0] = M;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) F[1 + d] = p_f * n[d] + dp * c[d] + M * uf[d] + mdot_c * du[d];
-  F[4] = M * h_f + mdot_c * dH;
-}
-
-// Compact closures (IdealGasSolverFlux.hpp:93-215), subtracted from F.
-// The closures use the two cells' properties and gradients only through
-// their sums: vs holds V_a + V_b field by field (same IEEE sums as the
-// reference's a + b forms, addition being commutative).
-__device__ __forceinline__ void compact_flux_add(Flux& F, const double un_[3], double area, double aod,
-                                                 double delta, const LRec& a, const LRec& b, const VRec& vs,
-                                                 const double uf[3], double h_f) {
-  const double half_aod = 0.5 * aod;
-  const double mu_area = 0.5 * vs.mu_total * area;
-  const double mu_aod = vs.mu_total * half_aod;
-  const double k_aod = vs.loc_total * half_aod;
-  const double hua = 0.5 * (a.u[0] * a.u[0] + a.u[1] * a.u[1] + a.u[2] * a.u[2]);
-  const double hub = 0.5 * (b.u[0] * b.u[0] + b.u[1] * b.u[1] + b.u[2] * b.u[2]);
-  const double d_half_usq = hub - hua;
   const double dh = b.h - a.h;
-  double una = 0.0, unb = 0.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    una += a.u[d] * un_[d];
-    unb += b.u[d] * un_[d];
-  }
-  const double dun = unb - una;
-  const double dun_3 = dun * (1.0 / 3.0);
-  const double dun2_6 = (unb * unb - una * una) * (1.0 / 6.0);
   const double dp = b.p - a.p;
-  const double fgr_f = 0.5 * vs.fgr;
   const double rho_m = 0.5 * (b.rho + a.rho);
-  const double un_m = 0.5 * (una + unb);
   const double c_m = 0.5 * (a.sos + b.sos);
-  const double mach_n = fabs(un_m) * rcp_nr(c_m);
   const double drho = b.rho - a.rho;
-  const double lf = fmin(fgr_f * mach_n, 0.5) * (c_m + fabs(un_m)) * area;
+  // Gibbs Lax-Friedrichs dissipation
+  const double aun = fabs(un_m);
+  const double lf = fmin(0.5 * vs.fgr * (aun * rcp_nr(c_m)), 0.5) * (c_m + aun) * area;
   const double lf_drho = lf * drho;
   const double lf_rho = lf * rho_m;
-  double ap = 0.5 * vs.a_sgs * delta * area;
-  ap += vs.symp * half_aod;
-  const double ap_dp = ap * dp;
-
-  F.rho -= lf_drho + ap_dp;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    F.ru[d] -= mu_aod * (b.u[d] - a.u[d] + dun_3 * un_[d]);
-    F.ru[d] -= lf_drho * uf[d];
-    F.ru[d] -= lf_rho * dun * un_[d];
-    F.ru[d] -= uf[d] * ap_dp;
-  }
-  F.rE -= mu_aod * (d_half_usq + dun2_6);
-  double hs = vs.symh * rho_m * fabs(un_m) * half_aod;
-  hs = fmax(hs - k_aod, 0.0);
-  F.rE -= (k_aod + hs) * dh;
-  F.rE -= ap_dp * h_f;
-  const double pva = a.p * a.sp_vol;
-  const double pvb = b.p * b.sp_vol;
-  const double pv_m = 0.5 * (pva + pvb);
-  const double de = dh - (pvb - pva);
-  F.rE -= lf_drho * (h_f - pv_m);
-  F.rE -= lf_rho * de;
-  F.rE -= lf_rho * un_m * dun;
+  // acoustic SGS
+  const double ap_dp = (0.5 * vs.a_sgs * delta * area + vs.symp * half_aod) * dp;
+  // the viscous stress's part along the gradients
   double gn[3];
-  double gnn_3 = 0.0, div_23 = 0.0;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    gn[k] = 0.5 * (vs.g[k] * un_[0] + vs.g[3 + k] * un_[1] + vs.g[6 + k] * un_[2]);
-    gnn_3 += gn[k] * un_[k];
-    div_23 += vs.g[4 * k];
-  }
-  div_23 *= (1.0 / 3.0);
-  gnn_3 *= (1.0 / 3.0);
+  for (int k = 0; k < 3; ++k) gn[k] = 0.5 * (vs.g[k] * un_[0] + vs.g[3 + k] * un_[1] + vs.g[6 + k] * un_[2]);
+  const double gnn_3 = (gn[0] * un_[0] + gn[1] * un_[1] + gn[2] * un_[2]) * (1.0 / 3.0);
+  const double div_23 = (vs.g[0] + vs.g[4] + vs.g[8]) * (1.0 / 3.0);
+  const double trace = gnn_3 + div_23;
+  const double m = lf_drho + ap_dp;
+  // along the normal: mu_aod dun/3 + lf_rho dun - mu_area trace
+  const double kn = (mu_aod * (1.0 / 3.0) + lf_rho) * dun - mu_area * trace;
+  acc[0] += m;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double t = (gn[d] - un_[d] * (gnn_3 + div_23)) * mu_area;
-    F.ru[d] -= t;
-    F.rE -= uf[d] * t;
+    acc[1 + d] += mu_aod * du[d];
+    acc[1 + d] += m * uf[d];
+    acc[1 + d] += kn * un_[d];
+    acc[1 + d] += mu_area * gn[d];
   }
+  const double hs = fmax(vs.symh * rho_m * aun * half_aod - k_aod, 0.0);
+  const double pva = a.p * a.sp_vol, pvb = b.p * b.sp_vol;
+  const double de = dh - (pvb - pva);
+  const double ufgn = uf[0] * gn[0] + uf[1] * gn[1] + uf[2] * gn[2];
+  double e = mu_aod * (ufdu + un_m * dun * (1.0 / 3.0));
+  e += (k_aod + hs) * dh;
+  e += m * h_f;
+  e -= lf_drho * (0.5 * (pva + pvb));
+  e += lf_rho * (de + un_m * dun);
+  e += mu_area * (ufgn - un_m * trace);
+  acc[4] += e;
+  return -m;
 }
 
 // ===========================================================================
@@ -389,211 +368,234 @@ __device__ __forceinline__ void compact_flux_add(Flux& F, const double un_[3], d
 // ===========================================================================
 
 
-// Every step kernel walks a work list of items (at most kItemCells cells of
-// one case each) with a grid-stride loop.  A kernel that puts G lanes on a
-// cell runs kThreads(G) = min(256, G*kItemCells) threads per CTA and splits
-// an item into kRounds(G) rounds of kThreads/G cells; one round is the unit a
-// CTA takes from the list.  Inside the loop `m`, `s` are the item's case mesh
-// and state, `i` the cell, `lane` the lane in the cell's group and `valid`
-// whether the cell exists (items are often shorter than a round).
+// The staged kernels walk a work list of items (at most kItemCells cells of
+// one case each) with a grid-stride loop, one item per CTA.  Several warps
+// share a slice's rows (lane i of each works on the slice's cell i): the CTA's
+// warps are dealt to at most kWarps/G slices at a time, so a full item has G
+// warps per slice ("lanes per cell") and a short one, in a small mesh, more.
+// Inside the loops `m`, `s` are the item's case mesh and state, `i` the cell,
+// `loc_` its index in the item, `part_` of `parts_` the warp's share of the
+// rows, and `valid` whether the cell exists.
+template <int G>
+__host__ __device__ constexpr int kWarps() {
+  return G == 1 ? 4 : G <= 8 ? 8 : G;
+}
 template <int G>
 __host__ __device__ constexpr int kThreads() {
-  return G * kItemCells >= 256 ? 256 : G * kItemCells;
+  return 32 * kWarps<G>();
 }
-template <int G>
-__host__ __device__ constexpr int kRounds() {
-  return (G * kItemCells + kThreads<G>() - 1) / kThreads<G>();
+// shared memory per warp for the sums of NV values of type T over the parts
+template <class T>
+__host__ __device__ constexpr int kSumBytes(int NV) {
+  return NV * 32 * int(sizeof(T));
 }
+// max_u, max_cu: the largest extended and compact unions of the launch's items
+// (the planes' length in shared memory)
 #define CASE_ARGS                                                              \
   const CaseDev* __restrict__ cases, const Item* __restrict__ items,           \
-      const int* __restrict__ nitems, const CaseDev dcase
-// DIRECT (a template parameter of every step kernel): one case passed by value
-// in `dcase`, items read from its mesh's own item table.
-#define ITEM_LOOP_BEGIN(G)                                                     \
-  constexpr int kR_ = kRounds<G>();                                            \
-  const int n_work_ = (DIRECT ? dcase.nitems : *nitems) * kR_;                 \
-  for (int v_ = blockIdx.x; v_ < n_work_; v_ += gridDim.x) {                   \
-    const Item it_ = DIRECT ? dcase.m.items[v_ / kR_] : items[v_ / kR_];       \
-    const int sub_ = v_ % kR_;                                                 \
-    const MeshDev& m = DIRECT ? dcase.m : cases[it_.c].m;                      \
-    const StateDev& s = DIRECT ? dcase.s : cases[it_.c].s;                     \
-    {                                                                          \
-      const int loc_ = sub_ * (kThreads<G>() / (G)) + int(threadIdx.x) / (G);  \
-      const int i = it_.cell0 + loc_;                                          \
-      const int lane = int(threadIdx.x) & ((G) - 1);                           \
-      const bool valid = loc_ < it_.ncell;
+      const int* __restrict__ nitems, const CaseDev dcase, const int max_u, const int max_cu
 #define CASE_PH (DIRECT ? dcase.ph : cases[it_.c].ph)
 #define CASE_NITEMS (DIRECT ? dcase.nitems : cases[it_.c].nitems)
-#define ITEM_LOOP_END \
-  }                   \
-  }
-
-// The face-flux kernels take a whole item per CTA (256 threads): they stage
-// the item's neighbour records in shared memory, then run its rounds.  The
-// entry streams of the round ahead (the next item's first round during the
-// last one) are prefetched into L2 by the bulk-copy engine meanwhile;
-// PREFETCH(item, mesh, round) names the kernel's stream.
-#define STAGED_LOOP_BEGIN(PREFETCH)                                            \
+// DIRECT (a template parameter of every step kernel): one case passed by value
+// in `dcase`, items read from its mesh's own item table.
+#define STAGED_LOOP_BEGIN(G)                                                   \
   const int n_items_ = DIRECT ? dcase.nitems : *nitems;                        \
-  if (blockIdx.x < n_items_) {                                                 \
-    const Item f_ = DIRECT ? dcase.m.items[blockIdx.x] : items[blockIdx.x];    \
-    PREFETCH(f_, (DIRECT ? dcase.m : cases[f_.c].m), 0);                       \
-  }                                                                            \
   for (int v_ = blockIdx.x; v_ < n_items_; v_ += gridDim.x) {                  \
     const Item it_ = DIRECT ? dcase.m.items[v_] : items[v_];                   \
     const MeshDev& m = DIRECT ? dcase.m : cases[it_.c].m;                      \
-    const StateDev& s = DIRECT ? dcase.s : cases[it_.c].s;
-#define STAGED_ROUNDS_BEGIN(G, PREFETCH)                                       \
-    for (int sub_ = 0; sub_ < (kItemCells * (G) + 255) / 256; ++sub_) {        \
-      if ((sub_ + 1) * (256 / (G)) < it_.ncell) {                              \
-        PREFETCH(it_, m, sub_ + 1);                                            \
-      } else if ((sub_ == 0 || sub_ * (256 / (G)) < it_.ncell) &&              \
-                 v_ + int(gridDim.x) < n_items_) {                             \
-        const Item n_ = DIRECT ? dcase.m.items[v_ + gridDim.x] : items[v_ + gridDim.x]; \
-        PREFETCH(n_, (DIRECT ? dcase.m : cases[n_.c].m), 0);                   \
-      }                                                                        \
-      const int loc_ = sub_ * (256 / (G)) + int(threadIdx.x) / (G);            \
-      const int i = it_.cell0 + loc_;                                          \
-      const int lane = int(threadIdx.x) & ((G) - 1);                           \
-      const bool valid = loc_ < it_.ncell;
-#define STAGED_ROUNDS_END }
+    const StateDev& s = DIRECT ? dcase.s : cases[it_.c].s;                     \
+    const int slice0_ = it_.cell0 / kSlice;                                    \
+    const int nsl_ = ((it_.cell0 & (kSlice - 1)) + it_.ncell + kSlice - 1) / kSlice; \
+    const int spr_ = min(nsl_, kWarps<G>() / (G));                             \
+    const int parts_ = kWarps<G>() / spr_;                                     \
+    const int part_ = (int(threadIdx.x) >> 5) % parts_;                        \
+    const int sub_ = (int(threadIdx.x) >> 5) / parts_;
+#define SLICES_BEGIN(G)                                                        \
+    for (int t_ = 0; t_ < nsl_; t_ += spr_) {                                  \
+      const int slice_ = slice0_ + t_ + sub_;                                  \
+      const int i = slice_ * kSlice + (int(threadIdx.x) & 31);                 \
+      const int loc_ = i - it_.cell0;                                          \
+      const bool valid = sub_ < spr_ && t_ + sub_ < nsl_ && loc_ >= 0 && loc_ < it_.ncell;
+#define SLICES_END }
 #define STAGED_LOOP_END \
     __syncthreads();    \
   }
+// Begin this warp's slice of the round that starts with the item's slice T.
+#define ROWS_START(ROWS_OF, COUNT, IDX, BASE, T)                               \
+  {                                                                            \
+    const int sl_ = slice0_ + (T) + sub_, ln_ = int(threadIdx.x) & 31;         \
+    const int lc_ = sl_ * kSlice + ln_ - it_.cell0;                            \
+    rows.left = 0;                                                             \
+    if (sub_ < spr_ && (T) + sub_ < nsl_) {                                    \
+      const int f_ = __ldg((ROWS_OF) + sl_);                                   \
+      const bool v_ = lc_ >= 0 && lc_ < it_.ncell;                             \
+      rows.start(BASE, IDX, f_, __ldg((ROWS_OF) + sl_ + 1) - f_,               \
+                 v_ ? int(m.cnt[sl_ * kSlice + ln_].COUNT) : 0, part_, parts_); \
+    }                                                                          \
+  }
 
-// calcRhsBase, cell-centric, in two passes over each cell's face list, a
-// group of G lanes per cell (lane l takes entries l, l+G, ...; the group's
-// partial sums are combined by a fixed butterfly):
+// Sum (MAXFIRST: the first value's maximum) of each lane's NV values over the
+// warps of its slice, in part order, left in part 0, through `bytes` (>= 32 NV
+// values) of shared memory per warp at `area`, which nothing else may be using.
+// All threads of the CTA call it; `again` (uniform) says that another round
+// follows.
+template <int NV, bool MAXFIRST = false, class T>
+__device__ __forceinline__ void combine_parts(T (&v)[NV], void* area, int bytes, int part, int parts, bool again) {
+  if (parts > 1) {
+    const int lane = int(threadIdx.x) & 31;
+    char* mine = static_cast<char*>(area) + (int(threadIdx.x) >> 5) * bytes;
+    __syncwarp();
+    if (part > 0) {
+      T* w = reinterpret_cast<T*>(mine) + lane;
+#pragma unroll
+      for (int c = 0; c < NV; ++c) w[c * 32] = v[c];
+    }
+    __syncthreads();
+    if (part == 0) {
+#pragma unroll 1
+      for (int p = 1; p < parts; ++p) {
+        const T* w = reinterpret_cast<const T*>(mine + p * bytes) + lane;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) v[c] = (MAXFIRST && c == 0) ? fmax(v[c], w[0]) : v[c] + w[c * 32];
+      }
+    }
+    if (again) __syncthreads();
+  }
+}
+
+// calcRhsBase, cell-centric, in two passes over each cell's face list:
 //   k_rhs_ext : rhs[i] = -sum over all of i's extended faces of the skew +
 //               symmetric flux F(i -> j)
 //   k_rhs_comp: rhs[i] -= sum over i's compact faces of the viscous/dissipation
 //               closure
 // Every face is evaluated by each of its two cells with the orientation
 // reversed (n -> -n, unit_n -> -unit_n, c kept), which gives the negated flux.
+//
+// k_rhs_ext streams 50 B per directed entry (about 80 a cell) and is bound by
+// HBM: 128^3 jittered cells 1.44 ms, 6.0 TB/s of rows (with an entry's six values
+// in planes of their own and G neighbouring lanes per cell, whose sums 40
+// shuffles a cell combined, 1.73 ms; 200^3 7.95 ms, where each CTA's seven
+// streams also missed the TLB).  A ring of rows in shared memory, filled by
+// bulk or per-thread asynchronous copies, covers the L2 latency better but
+// costs instructions and CTAs: 1.93 and 1.62 ms.
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256, 3) k_rhs_ext(CASE_ARGS, int stage) {
+__global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_rhs_ext(CASE_ARGS, int stage) {
   extern __shared__ int4 smem[];
-#define PF_EXT(it, mm, r) prefetch_round<false>(mm, mm.en, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_EXT)
-  stage_records<4>(smem, s.L, it_, m.hcell + it_.hoff, it_.nh);
+  int4* sE = smem + kWarps<G>() * kSumBytes<double>(5) / 16;
+  STAGED_LOOP_BEGIN(G)
+  Rows<1536, double2, 3> rows;
+  ROWS_START(m.erow, x, m.lidx, m.en, 0)
+  double* const mf = DIRECT ? s.mf : nullptr;  // (a batch's cases carry no scalars)
+  const int pl = plane_len(max_u, kEChunks);
+  stage_records<kEChunks, 4>(sE, pl, s.L, it_, m.hcell + it_.hoff, it_.nh);
+  const double K = CASE_PH.gamma * CASE_PH.invgm1;
   stage_wait();
-  const long long E = m.E;
-  STAGED_ROUNDS_BEGIN(G, PF_EXT)
-  long long b = 0, e = 0;
-  LRec Li;
+  SLICES_BEGIN(G)
+  ERec Ei;
+  double hi = 0.0;
   if (valid) {
-    b = m.off[i];
-    e = m.off[i + 1];
-    smem_L(smem, loc_, Li);
+    smem_E(sE, pl, loc_, Ei);
+    hi = K * (Ei.p * Ei.v);
   }
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (long long k = b + lane; k < e; k += G) {
-    const int jl = __ldg(m.lidx + k);
-    const double* g = m.en + k;
-    const double n[3] = {__ldg(g), __ldg(g + E), __ldg(g + 2 * E)};
-    const double c[3] = {__ldg(g + 3 * E), __ldg(g + 4 * E), __ldg(g + 5 * E)};
-    LRec Lj;
-    smem_L(smem, jl, Lj);
-    double F[5];
-    ext_flux(F, n, c, Li, Lj);
-    if (s.mf) s.mf[k] = F[0];  // mf[ief] of calcRhsBase, for calcRhsScalars
-#pragma unroll
-    for (int q = 0; q < 5; ++q) acc[q] -= F[q];
+  size_t k = 0;  // the entry's place in mf
+  if (mf && valid) k = (size_t(__ldg(m.erow + slice_)) + part_) * 32 + (threadIdx.x & 31);
+#pragma unroll 1
+  while (rows.left > 0) {
+    double2 g[3];
+    const int jl = rows.next(parts_, g);
+    ERec Ej;
+    smem_E(sE, pl, jl, Ej);
+    const double n[3] = {g[0].x, g[0].y, g[1].x}, c[3] = {g[1].y, g[2].x, g[2].y};
+    const double M = ext_flux_sub(acc, n, c, Ei, hi, Ej, K);
+    if (mf) {  // mf[ief] of calcRhsBase, for calcRhsScalars
+      mf[k] = M;
+      k += 32 * parts_;
+    }
   }
-#pragma unroll
-  for (int c = 0; c < 5; ++c) acc[c] = group_sum<G>(acc[c]);
-  if (valid) {
+  combine_parts(acc, smem, kSumBytes<double>(5), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
     double* r = s.rhs + size_t(stage) * 5 * m.N;
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-      if (c % G == lane) r[size_t(c) * m.N + i] = acc[c];
+    for (int c = 0; c < 5; ++c) r[size_t(c) * m.N + i] = acc[c];
   }
-  STAGED_ROUNDS_END
+  if (t_ + spr_ < nsl_) ROWS_START(m.erow, x, m.lidx, m.en, t_ + spr_)
+  SLICES_END
   STAGED_LOOP_END
-#undef PF_EXT
 }
 
-// Two CTAs per SM: the closure needs about 126 registers per thread, and at
-// three CTAs per SM (80 registers) it spills ~200 B per thread to local
-// memory, which measured 1.5x slower on the jittered 128^3 mesh.
+// 12 chunks of 16 bytes come from shared memory per entry besides its 50 B row,
+// and about 110 FP64 instructions follow: 128^3 0.88 ms (1.02 with G
+// neighbouring lanes per cell), 16 warps an SM at 128 registers.
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256, 2) k_rhs_comp(CASE_ARGS, int stage) {
+__global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 3 : G <= 8 ? 2 : 1) k_rhs_comp(CASE_ARGS, int stage) {
   extern __shared__ int4 smem[];
-#define PF_COMP(it, mm, r) prefetch_round<true>(mm, mm.qg, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_COMP)
-  const int nu = it_.ncell + it_.nch;
-  int4* sV = smem + swz_chunks<4>(nu);
-  stage_records<4>(smem, s.L, it_, m.chcell + it_.choff, it_.nch);
-  stage_records<8>(sV, s.V, it_, m.chcell + it_.choff, it_.nch);
+  int4* sL = smem + kWarps<G>() * kSumBytes<double>(5) / 16;
+  STAGED_LOOP_BEGIN(G)
+  Rows<1536, double2, 3> rows;
+  ROWS_START(m.qrow, y, m.clidx, m.qg, 0)
+  double* const mf = DIRECT ? s.mf : nullptr;
+  const int pl = plane_len(max_cu, 4), pv = plane_len(max_cu, 8);
+  int4* sV = sL + 4 * pl;
+  stage_records<4, 4>(sL, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
+  stage_records<8, 8>(sV, pv, s.V, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
-  const long long Q = m.Q;
-  STAGED_ROUNDS_BEGIN(G, PF_COMP)
-  long long q0 = 0, q1 = 0;
+  SLICES_BEGIN(G)
   LRec Li;
-  if (valid) {
-    q0 = m.qoff[i];
-    q1 = m.qoff[i + 1];
-    smem_L(smem, loc_, Li);
-  }
+  if (valid) smem_L(sL, pl, loc_, Li);
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (long long q = q0 + lane; q < q1; q += G) {
-    const int jl = __ldg(m.clidx + q);
-    const double* h = m.qg + q;
-    const double un[3] = {__ldg(h), __ldg(h + Q), __ldg(h + 2 * Q)};
-    const double area = __ldg(h + 3 * Q), aod = __ldg(h + 4 * Q), delta = __ldg(h + 5 * Q);
+  size_t q = 0;  // the entry's place in qmap
+  if (mf && valid) q = (size_t(__ldg(m.qrow + slice_)) + part_) * 32 + (threadIdx.x & 31);
+#pragma unroll 1
+  while (rows.left > 0) {
+    double2 h[3];
+    const int jl = rows.next(parts_, h);
     LRec Lj;
-    smem_L(smem, jl, Lj);
+    smem_L(sL, pl, jl, Lj);
     VRec Vs;
-    smem_V_sum(sV, loc_, jl, Vs);
-    // face averages of the skew flux (IdealGasSolverFlux.hpp:23-37)
-    double uf[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) uf[d] = 0.5 * (Li.u[d] + Lj.u[d]);
-    const double uaub = Li.u[0] * Lj.u[0] + Li.u[1] * Lj.u[1] + Li.u[2] * Lj.u[2];
-    const double h_f = 0.5 * ((Lj.h + Li.h) + uaub);
-    Flux F;
-    F.rho = 0.0; F.ru[0] = F.ru[1] = F.ru[2] = 0.0; F.rE = 0.0;
-    compact_flux_add(F, un, area, aod, delta, Li, Lj, Vs, uf, h_f);
-    // the closure's part of the face's mass flux (compact entries are the
-    // first entries of the cell's extended list)
-    if (s.mf) s.mf[m.off[i] + (q - q0)] += F.rho;
-    acc[0] -= F.rho;
-    acc[1] -= F.ru[0];
-    acc[2] -= F.ru[1];
-    acc[3] -= F.ru[2];
-    acc[4] -= F.rE;
+    smem_V_sum(sV, pv, loc_, jl, Vs);
+    const double un[3] = {h[0].x, h[0].y, h[1].x};
+    const double dm = compact_flux_add(acc, un, h[1].y, h[2].x, h[2].y, Li, Lj, Vs);
+    if (mf) {  // the closure's part of the face's mass flux
+      mf[(size_t(__ldg(m.erow + slice_)) + __ldg(m.qmap + q)) * 32 + (threadIdx.x & 31)] += dm;
+      q += 32 * parts_;
+    }
   }
-#pragma unroll
-  for (int c = 0; c < 5; ++c) acc[c] = group_sum<G>(acc[c]);
-  if (valid && q1 > q0) {
+  combine_parts(acc, smem, kSumBytes<double>(5), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
     double* r = s.rhs + size_t(stage) * 5 * m.N;
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-      if (c % G == lane) r[size_t(c) * m.N + i] += acc[c];
+    for (int c = 0; c < 5; ++c) r[size_t(c) * m.N + i] += acc[c];
   }
-  STAGED_ROUNDS_END
+  if (t_ + spr_ < nsl_) ROWS_START(m.qrow, y, m.clidx, m.qg, t_ + spr_)
+  SLICES_END
   STAGED_LOOP_END
-#undef PF_COMP
 }
 
-// calcRhsScalars (IdealGasSolver.cpp:537-693), cell-centric over each
-// cell's extended entries after both face kernels have left the entries'
-// mass fluxes in mf: rhs_sc[i] = -sum over the entries of
-// 0.5 (sc_i + sc_j) mf_ij, minus, on compact entries, the diffusive
-// -d_coeff (sc_j - sc_i) with d_coeff = 0.5 (loc_total_i + loc_total_j)
-// area_over_delta (unity Lewis number; loc_total = loc_lam + loc_sgs).
-// A group of G lanes per cell, lane l takes entries l, l+G, ...; partial
-// sums are combined by the fixed butterfly (deterministic).  The neighbour's
-// scalars and properties are gathered from global memory (scalar transport
-// runs on single-case solvers only).  MIX: the mixed-precision form, whose
-// mass fluxes come from the FP32 flux arithmetic and whose properties and
-// compact geometry are the FP32 records; scalars, fluxes and sums stay FP64.
-template <int G, bool MIX>
-__global__ void __launch_bounds__(256) k_rhs_sc(const CaseDev c, int stage) {
+// The cell behind a compact local index of item `it`: its own cells first,
+// then the halo it lists.
+__device__ __forceinline__ int comp_neighbour(const MeshDev& m, const Item& it, int jl) {
+  return (jl < it.ncell) ? it.cell0 + jl : __ldg(m.chcell + it.choff + jl - it.ncell);
+}
+
+// calcRhsScalars (IdealGasSolver.cpp:537-693), cell-centric after both face
+// kernels have left the entries' mass fluxes in mf: rhs_sc[i] = -sum over the
+// extended entries of 0.5 (sc_i + sc_j) mf_ij, plus on compact entries the
+// diffusive d_coeff (sc_j - sc_i) with d_coeff = 0.5 (loc_total_i +
+// loc_total_j) area_over_delta (unity Lewis number; loc_total = loc_lam +
+// loc_sgs).  One CTA per slice, its P warps share the rows as in the face
+// kernels.  The neighbour's scalars and properties are gathered from global
+// memory (scalar transport runs on single-case solvers only).  MIX: the
+// mixed-precision form, whose mass fluxes come from the FP32 flux arithmetic
+// and whose properties and compact geometry are the FP32 records; scalars,
+// fluxes and sums stay FP64.
+template <int P, bool MIX>
+__global__ void __launch_bounds__(32 * P) k_rhs_sc(const CaseDev c, int stage) {
+  __shared__ double red[(P - 1) * kMaxScalars * 32];
   const MeshDev& m = c.m;
   const StateDev& s = c.s;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = t / G, lane = t & (G - 1);
+  const int slice = blockIdx.x, part = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
+  const int i = slice * kSlice + lane;
   const bool valid = i < m.N;
   const int nsc = s.nsc;
   const size_t N = size_t(m.N);
@@ -603,50 +605,51 @@ __global__ void __launch_bounds__(256) k_rhs_sc(const CaseDev c, int stage) {
     acc[a] = 0.0;
     si[a] = (valid && a < nsc) ? s.sc[a * N + i] : 0.0;
   }
-  long long b = 0, e = 0;
-  int ncomp = 0;
+  int n = 0, nq = 0;
   double loc_i = 0.0;
   if (valid) {
-    b = m.off[i];
-    e = m.off[i + 1];
-    ncomp = int(m.qoff[i + 1] - m.qoff[i]);
+    n = m.cnt[i].x;
+    nq = m.cnt[i].y;
     loc_i = MIX ? double(s.VF[i].loc_total) : s.V[i].loc_total;
   }
-  const long long q0 = valid ? m.qoff[i] : 0;
-  for (long long k = b + lane; k < e; k += G) {
+  const size_t e0 = size_t(m.erow[slice]), q0 = size_t(m.qrow[slice]);
+  for (int r = part; r < n; r += P) {
+    const size_t k = (e0 + r) * 32 + lane;
     const int j = __ldg(m.nbr + k);
     const double mfk = s.mf[k];
-    const int tk = int(k - b);
-    double dc = 0.0;
-    if (tk < ncomp) {
-      if (MIX)
-        dc = 0.5 * (loc_i + double(s.VF[j].loc_total)) * double(__ldg(m.qg32 + 4 * m.Q + q0 + tk));
-      else
-        dc = 0.5 * (loc_i + s.V[j].loc_total) * __ldg(m.qg + 4 * m.Q + q0 + tk);
-    }
 #pragma unroll
-    for (int a = 0; a < kMaxScalars; ++a) {
-      if (a < nsc) {
-        const double sj = s.sc[a * N + j];
-        double flux = 0.5 * (si[a] + sj) * mfk;
-        flux -= dc * (sj - si[a]);
-        acc[a] -= flux;
-      }
-    }
+    for (int a = 0; a < kMaxScalars; ++a)
+      if (a < nsc) acc[a] -= 0.5 * (si[a] + s.sc[a * N + j]) * mfk;
   }
+  for (int r = part; r < nq; r += P) {
+    const size_t q = (q0 + r) * 32 + lane, h = (q0 + r) * 192 + 128;  // area_over_delta
+    const int j = __ldg(m.nbr + (e0 + __ldg(m.qmap + q)) * 32 + lane);
+    const double dc = MIX ? 0.5 * (loc_i + double(s.VF[j].loc_total)) * double(__ldg(m.qg32 + h + 2 * lane))
+                          : 0.5 * (loc_i + s.V[j].loc_total) * __ldg(m.qg + h + 2 * lane);
 #pragma unroll
-  for (int a = 0; a < kMaxScalars; ++a) acc[a] = group_sum<G>(acc[a]);
-  if (valid && lane == 0) {
+    for (int a = 0; a < kMaxScalars; ++a)
+      if (a < nsc) acc[a] += dc * (s.sc[a * N + j] - si[a]);
+  }
+  if (part > 0) {
+#pragma unroll
+    for (int a = 0; a < kMaxScalars; ++a)
+      if (a < nsc) red[((part - 1) * kMaxScalars + a) * 32 + lane] = acc[a];
+  }
+  __syncthreads();
+  if (valid && part == 0) {
     double* r = s.rhs_sc + size_t(stage) * nsc * N;
 #pragma unroll
     for (int a = 0; a < kMaxScalars; ++a)
-      if (a < nsc) r[a * N + i] = acc[a];
+      if (a < nsc) {
+        for (int p = 0; p < P - 1; ++p) acc[a] += red[(p * kMaxScalars + a) * 32 + lane];
+        r[a * N + i] = acc[a];
+      }
   }
 }
 
 // packed primitive state of one cell (updateExtendedState); FP64 always,
 // rounded into the FP32 records for mixed-precision solvers
-__device__ __forceinline__ void write_prim(const Phys& ph, StateDev& s, int i, double rho, double u0,
+__device__ __forceinline__ void write_prim(const Phys& ph, const StateDev& s, int i, double rho, double u0,
                                            double u1, double u2, double rhoE, bool writeQ) {
   const double gm1 = ph.gamma - 1.0;
   const double Rgogm1 = ph.R * ph.gamma * (1.0 / gm1);
@@ -665,18 +668,24 @@ __device__ __forceinline__ void write_prim(const Phys& ph, StateDev& s, int i, d
   }
   double* L = reinterpret_cast<double*>(s.L + i);
   st4(L, u0, u1, u2, 1.0 / rho);
-  st4(L + 4, p, Rgogm1 * T, rho, sos);
+  st4(L + 4, p, rho, Rgogm1 * T, sos);
   if (writeQ) st4(s.Q + i, log(p * (1.0 / ph.p_ref)), p, 1.0 / rho, 1.0 / (ph.R * T));
 }
 
 // rk3Step (when nw > 0) fused with the packed-state update of the new state,
 // one thread per cell.  dt_arg < 0 takes each case's dt from its control block.
 template <bool DIRECT>
-__global__ void __launch_bounds__(256) k_rk_prim(CASE_ARGS, int nw, double w0, double w1, double w2,
+__global__ void __launch_bounds__(kItemCells) k_rk_prim(CASE_ARGS, int nw, double w0, double w1, double w2,
                                                  double dt_arg, int writeQ) {
-  ITEM_LOOP_BEGIN(1)
-  (void)lane;
-  if (valid) {
+  // a single case takes its cells in order, a batch's case its items
+  const int n_items_ = DIRECT ? 0 : *nitems;
+  for (int v_ = blockIdx.x; DIRECT ? v_ == int(blockIdx.x) : v_ < n_items_; v_ += gridDim.x) {
+    Item it_{};
+    if (!DIRECT) it_ = items[v_];
+    const MeshDev& m = DIRECT ? dcase.m : cases[it_.c].m;
+    const StateDev& s = DIRECT ? dcase.s : cases[it_.c].s;
+    const int i = DIRECT ? v_ * kItemCells + int(threadIdx.x) : it_.cell0 + int(threadIdx.x);
+    if (DIRECT ? i >= m.N : int(threadIdx.x) >= it_.ncell) continue;
     const Phys& ph = CASE_PH;
     double rho = s.rho[i], u0 = s.u0[i], u1 = s.u1[i], u2 = s.u2[i], rhoE = s.rhoE[i];
     if (nw > 0) {
@@ -713,38 +722,37 @@ __global__ void __launch_bounds__(256) k_rk_prim(CASE_ARGS, int nw, double w0, d
         *ph_ = (rho_old * *ph_ + tmp * v) * inv_rho;
       }
     }
-    StateDev sw = s;
-    write_prim(ph, sw, i, rho, u0, u1, u2, rhoE, writeQ != 0);
+    write_prim(ph, s, i, rho, u0, u1, u2, rhoE, writeQ != 0);
   }
-  ITEM_LOOP_END
 }
 
-// _calcCvGradRange over the compact CSR (the reference's cvocv order), one
-// item per CTA, a group of G lanes per cell; the velocities of the item's
-// compact-face union are staged in shared memory (the first 32 bytes of each
-// LRec) and read through the per-entry local index cglidx.
+// _calcCvGradRange over the compact stencil (the reference's cvocv); the
+// velocities of the item's compact-face union are staged in shared memory (the
+// first 32 bytes of each LRec) and read through the entries' local indices.
+// 128^3: 0.266 ms (0.345 with G neighbouring lanes per cell).
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256) k_grad(CASE_ARGS) {
+__global__ void __launch_bounds__(kThreads<G>()) k_grad(CASE_ARGS) {
   extern __shared__ int4 smem[];
-#define PF_GRAD(it, mm, r) prefetch_grad(mm, mm.gcx, mm.gcy, mm.gcz, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_GRAD)
-  stage_records<2, 4>(smem, s.L, it_, m.chcell + it_.choff, it_.nch);
+  STAGED_LOOP_BEGIN(G)
+  Rows<768, double, 3> rows;
+  ROWS_START(m.grow, z, m.cglidx, m.gc, 0)
+  const int pl = plane_len(max_cu, 2);
+  stage_records<2, 4>(smem, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
   const double2* su = reinterpret_cast<const double2*>(smem);
-  STAGED_ROUNDS_BEGIN(G, PF_GRAD)
-  long long b = 0, e = 0;
+  SLICES_BEGIN(G)
   double ui[3] = {0.0, 0.0, 0.0};
   if (valid) {
-    b = m.coff[i];
-    e = m.coff[i + 1];
-    const double2 a = su[swz<2>(loc_, 0)], c = su[swz<2>(loc_, 1)];
+    const double2 a = su[loc_], c = su[pl + loc_];
     ui[0] = a.x; ui[1] = a.y; ui[2] = c.x;
   }
   double g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long k = b + lane; k < e; k += G) {
-    const int jl = __ldg(m.cglidx + k);
-    const double cx = __ldg(m.gcx + k), cy = __ldg(m.gcy + k), cz = __ldg(m.gcz + k);
-    const double2 ja = su[swz<2>(jl, 0)], jb = su[swz<2>(jl, 1)];
+#pragma unroll 2
+  while (rows.left > 0) {
+    double c[3];
+    const int jl = rows.next(parts_, c);
+    const double cx = c[0], cy = c[1], cz = c[2];
+    const double2 ja = su[jl], jb = su[pl + jl];
     const double du[3] = {ja.x - ui[0], ja.y - ui[1], jb.x - ui[2]};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -753,26 +761,26 @@ __global__ void __launch_bounds__(256) k_grad(CASE_ARGS) {
       g[3 * d + 2] += cz * du[d];
     }
   }
-#pragma unroll
-  for (int c = 0; c < 9; ++c) g[c] = group_sum<G>(g[c]);
-  if (valid) {
-#pragma unroll
-    for (int c = 0; c < 9; ++c)
-      if (c % G == lane) s.V[i].g[c] = g[c];
+  combine_parts(g, smem + 2 * pl, kSumBytes<double>(9), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
+    double* P = reinterpret_cast<double*>(s.V + i);
+    st4(P + 4, g[0], g[1], g[2], g[3]);
+    st4(P + 8, g[4], g[5], g[6], g[7]);
+    P[12] = g[8];
   }
-  STAGED_ROUNDS_END
+  if (t_ + spr_ < nsl_) ROWS_START(m.grow, z, m.cglidx, m.gc, t_ + spr_)
+  SLICES_END
   STAGED_LOOP_END
-#undef PF_GRAD
 }
 
 // Last block of a once-per-step kernel: reduce the per-block CFL maxima and
 // NaN flags (fixed order) and update the control block: time/step advance
 // (mode bit 0) and the next dt from setDt's formula (mode bit 1).
-// Called by all 256 threads of that block.
+// Called by all threads of that block (a power of two, 512 at most).
 __device__ __noinline__ void finalize_ctl(Ctl* ctl, const double* red, int dt_mode, double dt_max, int mode,
                                           int nparts) {
-  __shared__ double fin_cfl[256];
-  __shared__ int fin_nan[256];
+  __shared__ double fin_cfl[512];
+  __shared__ int fin_nan[512];
   double mx = 0.0;
   int anynan = 0;
   for (int bb = threadIdx.x; bb < nparts; bb += blockDim.x) {
@@ -882,8 +890,7 @@ __device__ __forceinline__ int cell_props(const Phys& ph, const MeshDev& m, cons
   if (ph.diss_mode == CGX_DISS_ALL) fgr = 0.5;
   double* P = reinterpret_cast<double*>(s.V + i);
   st4(P, mu_lam + mu_sgs, loc_lam + loc_sgs, a_sgs, fgr);
-  reinterpret_cast<double2*>(P)[2] = make_double2(symh, symp);
-  P[15] = mu_lam;
+  st4(P + 12, g[8], symh, symp, mu_lam);
   return (rho != rho) || (Li.p != Li.p) || (T != T);
 }
 
@@ -902,89 +909,30 @@ __device__ __forceinline__ double cfl_bf(const MeshDev& m, int i, double u0, dou
   return c;
 }
 
-// Once per step: cell_props + calcCfl(NULL, 1.0) for the next step's dt +
-// checkForNans, one item per CTA, a group of G lanes per cell for the face
-// loops.  The Gibbs remainder reads the item's extended-face union of QRec
-// and the CFL sum its compact-face union of LRec, both staged in shared
-// memory.  Each item leaves one partial (CFL maximum, NaN flag); the last
+// The CTA's CFL maximum and NaN flag, left as the item's partial; the last
 // item of a case reduces them in item order and updates the control block.
-// mode bit 0: advance time/step by the dt just used; bit 1: set dt from CFL.
-template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256, 3) k_step_end(CASE_ARGS, int mode) {
-  extern __shared__ int4 smem[];
-  __shared__ double sh_cfl[256];
-  __shared__ int sh_nan[256];
+// Called by all threads of the CTA (a power of two, 512 at most).
+__device__ __forceinline__ void item_partial(double cmax, int anynan, const StateDev& s, const Phys& ph, int idx,
+                                             int np, int mode) {
+  __shared__ double sh_cfl[16];
+  __shared__ int sh_nan[16];
   __shared__ bool am_last;
-#define PF_END(it, mm, r) prefetch_end(mm, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_END)
-  const Phys& ph = CASE_PH;
-  const int nu = it_.ncell + it_.nh;
-  int4* sL = smem + swz_chunks<2>(nu);
-  stage_records<2>(smem, s.Q, it_, m.hcell + it_.hoff, it_.nh);
-  stage_records<4>(sL, s.L, it_, m.chcell + it_.choff, it_.nch);
-  stage_wait();
-  const long long Q = m.Q;
-  // limitAsgs's dt: this step's, or outside a step the control block's
-  const double dt_sgs = (mode & 1) ? s.ctl->dt : s.ctl->dt_sgs;
-  double cmax = 0.0;
-  int anynan = 0;
-  STAGED_ROUNDS_BEGIN(G, PF_END)
-  long long b = 0, e = 0, q0 = 0, q1 = 0;
-  LRec Li;
-  double4 qi = make_double4(0.0, 0.0, 0.0, 0.0);
-  if (valid) {
-    b = m.off[i];
-    e = m.off[i + 1];
-    q0 = m.qoff[i];
-    q1 = m.qoff[i + 1];
-    smem_L(sL, loc_, Li);
-    qi = smem_Q(smem, loc_);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) cmax = fmax(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+  anynan = __any_sync(0xffffffffu, anynan);
+  const int warp = int(threadIdx.x) >> 5, nwarps = int(blockDim.x) >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    sh_cfl[warp] = cmax;
+    sh_nan[warp] = anynan;
   }
-  // ---- Gibbs remainder over the extended faces (a maximum: any order)
-  double vv2 = 0.0, cfl = 0.0;
-  for (long long k = b + lane; k < e; k += G) {
-    const double4 qj = smem_Q(smem, __ldg(m.lidx + k));
-    const double dp = qj.y - qi.y;
-    const double v_avg = 0.5 * (qi.z + qj.z);
-    const double beta = 0.5 * (qi.w + qj.w);
-    const double gr = qj.x - qi.x - v_avg * dp * beta;
-    vv2 = fmax(vv2, fabs(gr));
-  }
-  // ---- CFL over the compact faces
-  for (long long q = q0 + lane; q < q1; q += G) {
-    const int jl = __ldg(m.clidx + q);
-    const double* h = m.qg + q;
-    const double un[3] = {__ldg(h), __ldg(h + Q), __ldg(h + 2 * Q)};
-    const double area = __ldg(h + 3 * Q);
-    LRec Lj;
-    smem_L(sL, jl, Lj);
-    const double undA = 0.5 * area * ((Li.u[0] * un[0] + Li.u[1] * un[1] + Li.u[2] * un[2]) +
-                                      (Lj.u[0] * un[0] + Lj.u[1] * un[1] + Lj.u[2] * un[2]));
-    cfl += fabs(undA) + area * (0.5 * (Li.sos + Lj.sos));
-  }
-  vv2 = group_max<G>(vv2);
-  cfl = group_sum<G>(cfl);
-  if (valid && lane == 0) {
-    anynan |= cell_props(ph, m, s, i, Li, vv2, dt_sgs);
-    cfl += cfl_bf(m, i, Li.u[0], Li.u[1], Li.u[2], Li.sos);
-    cmax = fmax(cmax, cfl * (0.5 * 1.0 * __ldg(m.inv_vol + i)));
-  }
-  STAGED_ROUNDS_END
-  // ---- the item's partial; the last item of the case finalises
-  sh_cfl[threadIdx.x] = cmax;
-  sh_nan[threadIdx.x] = anynan;
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (int(threadIdx.x) < w) {
-      sh_cfl[threadIdx.x] = fmax(sh_cfl[threadIdx.x], sh_cfl[threadIdx.x + w]);
-      sh_nan[threadIdx.x] |= sh_nan[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    const int np = CASE_NITEMS;
-    s.red[it_.idx] = sh_cfl[0];
-    s.red[np + it_.idx] = double(sh_nan[0]);
+    for (int w = 1; w < nwarps; ++w) {
+      cmax = fmax(cmax, sh_cfl[w]);
+      anynan |= sh_nan[w];
+    }
+    s.red[idx] = cmax;
+    s.red[np + idx] = double(anynan != 0);
     __threadfence();
     const unsigned int done = atomicAdd(&s.ctl->blocks_done, 1u);
     am_last = (done == unsigned(np) - 1u);
@@ -992,10 +940,89 @@ __global__ void __launch_bounds__(256, 3) k_step_end(CASE_ARGS, int mode) {
   __syncthreads();
   if (am_last) {
     __threadfence();
-    finalize_ctl(s.ctl, s.red, ph.dt_mode, ph.dt_max, mode, CASE_NITEMS);
+    finalize_ctl(s.ctl, s.red, ph.dt_mode, ph.dt_max, mode, np);
   }
+}
+
+// Once per step: cell_props + calcCfl(NULL, 1.0) for the next step's dt +
+// checkForNans, one item per CTA.  The Gibbs remainder reads the item's
+// extended-face union of QRec and the CFL sum its compact-face union of LRec,
+// both staged in shared memory; the properties (logarithm, exponentials, square
+// roots in FP64) are then evaluated with every lane of part 0 on a cell of its
+// own.  128^3: 0.985 ms (1.17 with G neighbouring lanes per cell, one of which
+// evaluated the properties).  Faces and properties in two kernels, the latter
+// with a thread per cell at 24 warps an SM, took 1.05.
+// mode bit 0: advance time/step by the dt just used; bit 1: set dt from CFL.
+template <int G, bool DIRECT>
+__global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 5 : G <= 8 ? 3 : 1) k_step_end(CASE_ARGS, int mode) {
+  extern __shared__ int4 smem[];
+  int4* sQ = smem + kWarps<G>() * kSumBytes<double>(2) / 16;
+  STAGED_LOOP_BEGIN(G)
+  Rows<1536, double2, 2> rows;  // unit normals and areas
+  ROWS_START(m.qrow, y, m.clidx, m.qg, 0)
+  if (sub_ < spr_ && part_ == 0 && (threadIdx.x & 31) == 0) {
+    const int r0 = __ldg(m.erow + slice0_ + sub_), r1 = __ldg(m.erow + slice0_ + sub_ + 1);
+    prefetch_l2(m.lidx + size_t(r0) * kSlice, (long long)(r1 - r0) * kSlice * 2);
+  }
+  const Phys& ph = CASE_PH;
+  const int pq = plane_len(max_u, 2), pl = plane_len(max_cu, 4);
+  int4* sL = sQ + 2 * pq;
+  stage_records<2, 2>(sQ, pq, s.Q, it_, m.hcell + it_.hoff, it_.nh);
+  stage_records<4, 4>(sL, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
+  stage_wait();
+  // limitAsgs's dt: this step's, or outside a step the control block's
+  const double dt_sgs = (mode & 1) ? s.ctl->dt : s.ctl->dt_sgs;
+  double cmax = 0.0;
+  int anynan = 0;
+  SLICES_BEGIN(G)
+  int n = 0;
+  double4 qi = make_double4(0.0, 0.0, 0.0, 0.0);
+  const unsigned short* eidx = m.lidx + (threadIdx.x & 31);
+  if (valid) {
+    n = m.cnt[i].x;
+    eidx += size_t(__ldg(m.erow + slice_)) * 32;
+    qi = smem_Q(sQ, pq, loc_);
+  }
+  // ---- Gibbs remainder over the extended faces (a maximum: any order)
+  double v[2] = {0.0, 0.0};  // the remainder's maximum, the CFL sum
+  for (int r = part_; r < n; r += kIdxBatch * parts_) {
+    int jl[kIdxBatch];  // (past the last row: the cell itself, remainder zero)
+#pragma unroll
+    for (int b = 0; b < kIdxBatch; ++b) jl[b] = (r + b * parts_ < n) ? __ldg(eidx + (r + b * parts_) * 32) : loc_;
+#pragma unroll
+    for (int b = 0; b < kIdxBatch; ++b) {
+      const double4 qj = smem_Q(sQ, pq, jl[b]);
+      const double dp = qj.y - qi.y;
+      const double v_avg = 0.5 * (qi.z + qj.z);
+      const double beta = 0.5 * (qi.w + qj.w);
+      const double gr = qj.x - qi.x - v_avg * dp * beta;
+      v[0] = fmax(v[0], fabs(gr));
+    }
+  }
+  // ---- CFL over the compact faces
+  LRec Li;
+  if (valid) smem_L(sL, pl, loc_, Li);
+#pragma unroll 1
+  while (rows.left > 0) {
+    double2 h[2];
+    const int jl = rows.next(parts_, h);
+    LRec Lj;
+    smem_L(sL, pl, jl, Lj);
+    const double undA = 0.5 * h[1].y * ((Li.u[0] * h[0].x + Li.u[1] * h[0].y + Li.u[2] * h[1].x) +
+                                        (Lj.u[0] * h[0].x + Lj.u[1] * h[0].y + Lj.u[2] * h[1].x));
+    v[1] += fabs(undA) + h[1].y * (0.5 * (Li.sos + Lj.sos));
+  }
+  combine_parts<2, true>(v, smem, kSumBytes<double>(2), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
+    smem_L(sL, pl, loc_, Li);
+    anynan |= cell_props(ph, m, s, i, Li, v[0], dt_sgs);
+    const double cfl = v[1] + cfl_bf(m, i, Li.u[0], Li.u[1], Li.u[2], Li.sos);
+    cmax = fmax(cmax, cfl * (0.5 * 1.0 * __ldg(m.inv_vol + i)));
+  }
+  if (t_ + spr_ < nsl_) ROWS_START(m.qrow, y, m.clidx, m.qg, t_ + spr_)
+  SLICES_END
+  item_partial(cmax, anynan, s, ph, it_.idx, CASE_NITEMS, mode);
   STAGED_LOOP_END
-#undef PF_END
 }
 
 #include "cgx_mixed.cuh"
@@ -2251,48 +2278,61 @@ __global__ void k_field_in(int N, const int* __restrict__ perm, const double* __
   for (int c = 0; c < 5; ++c) field[size_t(c) * N + i] = src[5 * size_t(o) + c];
 }
 
-// Per-entry geometry planes from the per-face records: entry k of the
-// extended CSR reads face fid[k] (bit 31: the cell is the face's second cell,
-// normal negated); compact entry q = qoff[i] + t mirrors extended entry
-// off[i] + t (eofq[q]).  One thread per entry.
+// Fill the rows' geometry from the per-face records: fid / qfid hold each
+// entry's face (bit 31: the cell is the face's second cell, normal negated;
+// kNoFace: an empty lane, zeros).  One thread per entry.
 __global__ void k_expand_entries(long long E, long long Q, const int* __restrict__ fid,
-                                 const EFRec* __restrict__ ef, const CFRec* __restrict__ cf,
-                                 const long long* __restrict__ eofq, double* __restrict__ en,
-                                 double* __restrict__ qg) {
+                                 const int* __restrict__ qfid, const double* __restrict__ n_ef,
+                                 const double* __restrict__ c_ef, const CFRec* __restrict__ cf,
+                                 double2* __restrict__ en, double2* __restrict__ qg) {
   const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (k < E) {
     const int f = fid[k];
-    const EFRec r = ef[f & kFidMask];
+    const size_t a = 3 * size_t(f & kFidMask);
     const double sg = (f < 0) ? -1.0 : 1.0;
-    for (int d = 0; d < 3; ++d) {
-      en[d * E + k] = sg * r.n[d];
-      en[(3 + d) * E + k] = r.c[d];
-    }
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (f != kNoFace)
+      for (int d = 0; d < 3; ++d) {
+        v[d] = sg * n_ef[a + d];
+        v[3 + d] = 0.5 * c_ef[a + d];  // FlowSolver.hpp:2256-2259
+      }
+    double2* o = en + (k / 32) * 96 + (k & 31);
+    for (int c = 0; c < 3; ++c) o[32 * c] = make_double2(v[2 * c], v[2 * c + 1]);
   }
   if (k < Q) {
-    const int f = fid[eofq[k]];
-    const CFRec r = cf[f & kFidMask];
+    const int f = qfid[k];
+    CFRec r{};
+    if (f != kNoFace) r = cf[f & kFidMask];
     const double sg = (f < 0) ? -1.0 : 1.0;
-    for (int d = 0; d < 3; ++d) qg[d * Q + k] = sg * r.un[d];
-    qg[3 * Q + k] = r.area;
-    qg[4 * Q + k] = r.aod;
-    qg[5 * Q + k] = r.delta;
+    double2* o = qg + (k / 32) * 96 + (k & 31);
+    o[0] = make_double2(sg * r.un[0], sg * r.un[1]);
+    o[32] = make_double2(sg * r.un[2], r.area);
+    o[64] = make_double2(r.aod, r.delta);
+  }
+}
+
+// The global neighbour of every extended entry from its local index: the
+// item's own cells first, then its halo.  One CTA per item.
+__global__ void k_fill_nbr(MeshDev m, int* __restrict__ nbr) {
+  const Item it = m.items[blockIdx.x];
+  for (int t = threadIdx.x; t < it.ncell; t += blockDim.x) {
+    const int i = it.cell0 + t, n = m.cnt[i].x;
+    const size_t k0 = size_t(m.erow[i / kSlice]) * kSlice + (i & (kSlice - 1));
+    for (int r = 0; r < n; ++r) {
+      const int j = m.lidx[k0 + size_t(r) * kSlice];
+      nbr[k0 + size_t(r) * kSlice] = (j < it.ncell) ? it.cell0 + j : m.hcell[it.hoff + j - it.ncell];
+    }
   }
 }
 
 // FP32 copies of the entry geometry and gradient coefficients (mixed form)
 __global__ void k_geom32(long long ne, long long nq, long long nc, const double* __restrict__ en,
-                         const double* __restrict__ qg, const double* __restrict__ gx,
-                         const double* __restrict__ gy, const double* __restrict__ gz, float* en32,
-                         float* qg32, float* gx32, float* gy32, float* gz32) {
+                         const double* __restrict__ qg, const double* __restrict__ gc, float* en32, float* qg32,
+                         float* gc32) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t < ne) en32[t] = float(en[t]);
   if (t < nq) qg32[t] = float(qg[t]);
-  if (t < nc) {
-    gx32[t] = float(gx[t]);
-    gy32[t] = float(gy[t]);
-    gz32[t] = float(gz[t]);
-  }
+  if (t < nc) gc32[t] = float(gc[t]);
 }
 
 // calcCfl(cfl, dt) per cell (diagnostic; the stepping path uses k_step_end)
@@ -2313,12 +2353,15 @@ __global__ void k_cfl_cells(MeshDev m, StateDev s, const int* __restrict__ perm,
   };
   double ui[3], si;
   vel(i, ui, si);
-  const long long b = m.off[i], q0 = m.qoff[i], q1 = m.qoff[i + 1];
+  const int lane = i & (kSlice - 1), nq = m.cnt[i].y;
+  const size_t q0 = size_t(m.qrow[i / kSlice]);
+  const Item it = m.items[m.item_of[i]];
   double cfl = 0.0;
-  for (long long q = q0; q < q1; ++q) {
-    const int j = m.nbr[b + (q - q0)];
-    const double un[3] = {m.qg[q], m.qg[m.Q + q], m.qg[2 * m.Q + q]};
-    const double area = m.qg[3 * m.Q + q];
+  for (int r = 0; r < nq; ++r) {
+    const int j = comp_neighbour(m, it, m.clidx[(q0 + r) * 32 + lane]);
+    const double2* h = reinterpret_cast<const double2*>(m.qg) + (q0 + r) * 96 + lane;
+    const double un[3] = {h[0].x, h[0].y, h[32].x};
+    const double area = h[32].y;
     double uj[3], sj;
     vel(j, uj, sj);
     const double undA = 0.5 * area * ((ui[0] * un[0] + ui[1] * un[1] + ui[2] * un[2]) +
@@ -2400,17 +2443,21 @@ using uvec = std::vector<T, DefaultInit<T>>;
 // device copy of a host vector; large ones go through the pinned staging
 // buffers (asynchronous on the legacy default stream, which the set-up
 // kernels also use)
-template <class T, class A>
-int dupload(T** p, const std::vector<T, A>& v, size_t* acc, cgx_staging::Staging* st = nullptr) {
-  int rc = dalloc(p, v.size(), acc);
+template <class T>
+int dupload(T** p, const T* v, size_t n, cgx_staging::Staging* st, size_t* acc = nullptr) {
+  int rc = dalloc(p, n, acc);
   if (rc) return rc;
-  const size_t bytes = v.size() * sizeof(T);
+  const size_t bytes = n * sizeof(T);
   if (st && bytes >= (size_t(8) << 20)) {
-    CK(st->put(*p, v.data(), bytes));
-  } else if (!v.empty()) {
-    CK(cudaMemcpy(*p, v.data(), bytes, cudaMemcpyHostToDevice));
+    CK(st->put(*p, v, bytes));
+  } else if (n > 0) {
+    CK(cudaMemcpy(*p, v, bytes, cudaMemcpyHostToDevice));
   }
   return CGX_OK;
+}
+template <class T, class A>
+int dupload(T** p, const std::vector<T, A>& v, size_t* acc, cgx_staging::Staging* st = nullptr) {
+  return dupload(p, v.data(), v.size(), st, acc);
 }
 
 inline uint64_t spread3(uint64_t x) {  // 21 bits -> every third bit
@@ -2428,7 +2475,7 @@ inline uint64_t spread3(uint64_t x) {  // 21 bits -> every third bit
 struct cgx_mesh {
   int device = 0;
   int N = 0, ncv_g2 = 0;
-  long long nc_dir = 0;  // gradient entries (for the FP32 copies)
+  long long nq = 0, nc = 0;  // compact and gradient entries, empty lanes included
   bool have32 = false;
   std::vector<int> perm;  // new -> old
   MeshDev md{};
@@ -2445,9 +2492,9 @@ struct cgx_mesh {
   cgx_mesh_stats stats{};
 };
 
-// Lanes per cell of each face/gradient/step kernel.
+// Warps per slice (lanes per cell) of each face/gradient/step kernel.
 struct Tune {
-  int g_ext = 16, g_comp = 16, g_grad = 4, g_end = 4;
+  int g_ext = 2, g_comp = 2, g_grad = 2, g_end = 2;
 };
 
 // The source terms of a single-case solver (cgx_set_source,
@@ -2550,76 +2597,73 @@ int launch_check(const Runner& R, int nk) {
   return CGX_OK;
 }
 
-#define RARGS R.cases, R.items, R.nitems, R.dcase
+#define RARGS R.cases, R.items, R.nitems, R.dcase, R.max_union, R.max_cunion
 
-// rounds per item and CTAs for a kernel with G lanes per cell
-inline int rounds_host(int G) {
-  const int t = std::min(256, G * kItemCells);
-  return (G * kItemCells + t - 1) / t;
-}
-inline int grid_for(const Runner& R, int G) {
-  return R.nitems_host >= 0 ? std::max(1, R.nitems_host * rounds_host(G)) : R.grid;
-}
-// the face-flux kernels take one item per CTA
+// the staged kernels take one item per CTA
 inline int grid_staged(const Runner& R) { return R.nitems_host >= 0 ? std::max(1, R.nitems_host) : R.grid; }
 
-// dynamic shared memory of the staged face-flux kernels
+// dynamic shared memory of the staged kernels: the records, then the sums of
+// the warps that share a slice
+inline size_t planes(int n, int R) { return size_t(R) * plane_len(n, R) * 16; }
+template <int G>
 inline size_t smem_ext(const Runner& R) {
-  return size_t(R.prec == CGX_MIXED ? swz_chunks<2>(R.max_union) : swz_chunks<4>(R.max_union)) * 16;
+  return planes(R.max_union, R.prec == CGX_MIXED ? 2 : kEChunks) + kWarps<G>() * kSumBytes<double>(5);
 }
+template <int G>
 inline size_t smem_grad(const Runner& R) {
-  return size_t(R.prec == CGX_MIXED ? swz_chunks<1>(R.max_cunion) : swz_chunks<2>(R.max_cunion)) * 16;
+  return R.prec == CGX_MIXED ? planes(R.max_cunion, 1) + kWarps<G>() * kSumBytes<float>(9)
+                             : planes(R.max_cunion, 2) + kWarps<G>() * kSumBytes<double>(9);
 }
+template <int G>
 inline size_t smem_end(const Runner& R) {
-  return size_t(R.prec == CGX_MIXED ? swz_chunks<1>(R.max_union) + swz_chunks<2>(R.max_cunion)
-                                    : swz_chunks<2>(R.max_union) + swz_chunks<4>(R.max_cunion)) *
-         16;
+  const bool mix = R.prec == CGX_MIXED;
+  return planes(R.max_union, mix ? 1 : 2) + planes(R.max_cunion, mix ? 2 : 4) + kWarps<G>() * kSumBytes<double>(2);
 }
+template <int G>
 inline size_t smem_comp(const Runner& R) {
-  return size_t(R.prec == CGX_MIXED ? swz_chunks<2>(R.max_cunion) + swz_chunks<4>(R.max_cunion)
-                                    : swz_chunks<4>(R.max_cunion) + swz_chunks<8>(R.max_cunion)) *
-         16;
+  const bool mix = R.prec == CGX_MIXED;
+  return planes(R.max_cunion, mix ? 2 : 4) + planes(R.max_cunion, mix ? 4 : 8) + kWarps<G>() * kSumBytes<double>(5);
 }
 
 int enqueue_prim(const Runner& R, int nw, const double* w, double dt_arg, bool writeQ) {
+  const double w0 = w ? w[0] : 0.0, w1 = w ? w[1] : 0.0, w2 = w ? w[2] : 0.0;
   if (R.direct)
-    k_rk_prim<true><<<grid_for(R, 1), kThreads<1>(), 0, R.stream>>>(RARGS, nw, w ? w[0] : 0.0, w ? w[1] : 0.0,
-                                                                     w ? w[2] : 0.0, dt_arg, writeQ ? 1 : 0);
+    k_rk_prim<true><<<(R.dcase.m.N + kItemCells - 1) / kItemCells, kItemCells, 0, R.stream>>>(
+        RARGS, nw, w0, w1, w2, dt_arg, writeQ ? 1 : 0);
   else
-    k_rk_prim<false><<<grid_for(R, 1), kThreads<1>(), 0, R.stream>>>(RARGS, nw, w ? w[0] : 0.0, w ? w[1] : 0.0,
-                                                                      w ? w[2] : 0.0, dt_arg, writeQ ? 1 : 0);
+    k_rk_prim<false><<<R.grid, kItemCells, 0, R.stream>>>(RARGS, nw, w0, w1, w2, dt_arg, writeQ ? 1 : 0);
   return launch_check(R, 1);
 }
 
-// Lanes per cell of the group-per-cell kernels, chosen per mesh-size bucket
-// by autotune() (timed candidates, cached process-wide).
+// Warps per slice of the staged kernels, chosen per mesh-size bucket by
+// autotune() (timed candidates, cached process-wide).
 template <int G, bool MIX, bool DIRECT>
 void launch_grad_d(const Runner& R) {
   if (MIX)
-    k_grad_f<G, DIRECT><<<grid_staged(R), 256, smem_grad(R), R.stream>>>(RARGS);
+    k_grad_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_grad<G>(R), R.stream>>>(RARGS);
   else
-    k_grad<G, DIRECT><<<grid_staged(R), 256, smem_grad(R), R.stream>>>(RARGS);
+    k_grad<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_grad<G>(R), R.stream>>>(RARGS);
 }
 template <int G, bool MIX, bool DIRECT>
 void launch_ext_d(const Runner& R, int st) {
   if (MIX)
-    k_rhs_ext_f<G, DIRECT><<<grid_staged(R), 256, smem_ext(R), R.stream>>>(RARGS, st);
+    k_rhs_ext_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_ext<G>(R), R.stream>>>(RARGS, st);
   else
-    k_rhs_ext<G, DIRECT><<<grid_staged(R), 256, smem_ext(R), R.stream>>>(RARGS, st);
+    k_rhs_ext<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_ext<G>(R), R.stream>>>(RARGS, st);
 }
 template <int G, bool MIX, bool DIRECT>
 void launch_comp_d(const Runner& R, int st) {
   if (MIX)
-    k_rhs_comp_f<G, DIRECT><<<grid_staged(R), 256, smem_comp(R), R.stream>>>(RARGS, st);
+    k_rhs_comp_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_comp<G>(R), R.stream>>>(RARGS, st);
   else
-    k_rhs_comp<G, DIRECT><<<grid_staged(R), 256, smem_comp(R), R.stream>>>(RARGS, st);
+    k_rhs_comp<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_comp<G>(R), R.stream>>>(RARGS, st);
 }
 template <int G, bool MIX, bool DIRECT>
 void launch_end_d(const Runner& R, int mode) {
   if (MIX)
-    k_step_end_f<G, DIRECT><<<grid_staged(R), 256, smem_end(R), R.stream>>>(RARGS, mode);
+    k_step_end_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_end<G>(R), R.stream>>>(RARGS, mode);
   else
-    k_step_end<G, DIRECT><<<grid_staged(R), 256, smem_end(R), R.stream>>>(RARGS, mode);
+    k_step_end<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_end<G>(R), R.stream>>>(RARGS, mode);
 }
 
 // The staged kernels may use more than the default 48 KB of dynamic shared
@@ -2659,6 +2703,10 @@ int prepare_kernels(int device) {
   std::lock_guard<std::mutex> lk(g_smem_mu);
   if (device < 0 || device >= 64 || ((g_smem_done >> device) & 1ULL)) return CGX_OK;
   CK(cudaDeviceGetAttribute(&g_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  allow_smem_ext<1, true>();
+  allow_smem_ext<1, false>();
+  allow_smem_ext<2, true>();
+  allow_smem_ext<2, false>();
   allow_smem_ext<4, true>();
   allow_smem_ext<4, false>();
   allow_smem_ext<8, true>();
@@ -2667,6 +2715,8 @@ int prepare_kernels(int device) {
   allow_smem_ext<16, false>();
   allow_smem_ext<32, true>();
   allow_smem_ext<32, false>();
+  allow_smem_comp<1, true>();
+  allow_smem_comp<1, false>();
   allow_smem_comp<2, true>();
   allow_smem_comp<2, false>();
   allow_smem_comp<4, true>();
@@ -2687,6 +2737,8 @@ int prepare_kernels(int device) {
   allow_smem_grad<16, false>();
   allow_smem_end<1, true>();
   allow_smem_end<1, false>();
+  allow_smem_end<2, true>();
+  allow_smem_end<2, false>();
   allow_smem_end<4, true>();
   allow_smem_end<4, false>();
   allow_smem_end<8, true>();
@@ -2704,10 +2756,14 @@ void launch_grad(const Runner& R) {
 }
 template <int G, bool MIX>
 void launch_ext(const Runner& R, int st) {
+  if constexpr (G > 1)  // an item with a huge halo leaves room for few warps
+    if (smem_ext<G>(R) > size_t(g_smem_optin)) return launch_ext<1, MIX>(R, st);
   R.direct ? launch_ext_d<G, MIX, true>(R, st) : launch_ext_d<G, MIX, false>(R, st);
 }
 template <int G, bool MIX>
 void launch_comp(const Runner& R, int st) {
+  if constexpr (G > 1)  // an item with a huge halo leaves room for few warps
+    if (smem_comp<G>(R) > size_t(g_smem_optin)) return launch_comp<1, MIX>(R, st);
   R.direct ? launch_comp_d<G, MIX, true>(R, st) : launch_comp_d<G, MIX, false>(R, st);
 }
 template <int G, bool MIX>
@@ -2728,6 +2784,8 @@ void grad_g(const Runner& R, int G) {
 template <bool MIX>
 void ext_g(const Runner& R, int G, int st) {
   switch (G) {
+    case 1: launch_ext<1, MIX>(R, st); break;
+    case 2: launch_ext<2, MIX>(R, st); break;
     case 4: launch_ext<4, MIX>(R, st); break;
     case 8: launch_ext<8, MIX>(R, st); break;
     case 32: launch_ext<32, MIX>(R, st); break;
@@ -2737,6 +2795,7 @@ void ext_g(const Runner& R, int G, int st) {
 template <bool MIX>
 void comp_g(const Runner& R, int G, int st) {
   switch (G) {
+    case 1: launch_comp<1, MIX>(R, st); break;
     case 2: launch_comp<2, MIX>(R, st); break;
     case 4: launch_comp<4, MIX>(R, st); break;
     case 8: launch_comp<8, MIX>(R, st); break;
@@ -2747,6 +2806,7 @@ template <bool MIX>
 void end_g(const Runner& R, int G, int mode) {
   switch (G) {
     case 1: launch_end<1, MIX>(R, mode); break;
+    case 2: launch_end<2, MIX>(R, mode); break;
     case 4: launch_end<4, MIX>(R, mode); break;
     case 8: launch_end<8, MIX>(R, mode); break;
     default: launch_end<16, MIX>(R, mode); break;
@@ -2777,12 +2837,12 @@ int enqueue_grad(const Runner& R) { return grad_var(R, R.tune.g_grad); }
 // calcRhsScalars, once both face kernels have completed mf
 int enqueue_rhs_sc(const Runner& R, int stage0) {
   {
-    constexpr int G = 4;
-    const long long thr = (long long)R.dcase.m.N * G;
+    constexpr int P = 4;
+    const int slices = (R.dcase.m.N + kSlice - 1) / kSlice;
     if (R.prec == CGX_MIXED)
-      k_rhs_sc<G, true><<<int((thr + 255) / 256), 256, 0, R.stream>>>(R.dcase, stage0);
+      k_rhs_sc<P, true><<<slices, 32 * P, 0, R.stream>>>(R.dcase, stage0);
     else
-      k_rhs_sc<G, false><<<int((thr + 255) / 256), 256, 0, R.stream>>>(R.dcase, stage0);
+      k_rhs_sc<P, false><<<slices, 32 * P, 0, R.stream>>>(R.dcase, stage0);
     return launch_check(R, 1);
   }
 }
@@ -2970,7 +3030,8 @@ bool fixed_tune(Tune* t) {
       if (g == x) return true;
     return false;
   };
-  if (!ok(a, {4, 8, 16, 32}) || !ok(b, {2, 4, 8, 16}) || !ok(c, {1, 2, 4, 8, 16}) || !ok(d, {1, 4, 8, 16}))
+  if (!ok(a, {1, 2, 4, 8, 16, 32}) || !ok(b, {1, 2, 4, 8, 16}) || !ok(c, {1, 2, 4, 8, 16}) ||
+      !ok(d, {1, 2, 4, 8, 16}))
     return false;
   *t = Tune{a, b, c, d};
   return true;
@@ -3003,8 +3064,7 @@ int autotune(Runner& R, long long ncells) {
   Tune best = R.tune;
   float bt;
   int rc = CGX_OK;
-  const int ext_c[] = {4, 8, 16, 32}, comp_c[] = {2, 4, 8, 16}, grad_c[] = {1, 2, 4, 8, 16},
-            end_c[] = {1, 4, 8, 16};
+  const int ext_c[] = {1, 2, 4, 8, 16}, comp_c[] = {1, 2, 4, 8}, grad_c[] = {1, 2, 4, 8}, end_c[] = {1, 2, 4, 8};
   bt = 1e30f;
   for (int G : ext_c) {
     float ms;
@@ -3205,6 +3265,76 @@ extern "C" void cgx_params_default(cgx_params* p) {
   p->limit_asgs = 0;
 }
 
+// Cells per work item of a mesh of N cells.  Items of 128 have the smallest
+// halos and fullest rows; below about two of them per SM the items shrink to 64
+// and 32 cells, so that a small mesh still has an item for every SM, each item's
+// rows then split over more warps.  One FP64 step with items of 32 / 64 / 128
+// cells: 16^3 0.077 / 0.098 / 0.138 ms, 24^3 0.122 / 0.147 / 0.160; with 64 /
+// 128: 32^3 0.287 / 0.265 FP64 and 0.179 / 0.226 mixed.  A batch of many small
+// boxes fills the GPU either way and loses 4 % with the short items.
+static int item_cells(int N) {
+  for (int c = kItemCells; c > kSlice; c /= 2)
+    if ((long long)N >= 2LL * 148 * c) return c;
+  return kSlice;
+}
+
+// The order of a slice's entries: rows x 32 lanes, each lane's entries (the
+// range off[l], off[l+1] of idx) in any order, one per row from row 0 on.  The
+// 16-byte shared-memory reads of eight neighbouring lanes are served together
+// when they fall into different bank groups, and a record's bank group follows
+// from its local index modulo 8.  So for each row and each eight lanes this
+// takes, lane by lane, an entry of a class that the row's earlier lanes have
+// not taken, from the class the lane has most of; where a lane has none left,
+// one that shares a bank.
+namespace {
+class RowOrder {
+ public:
+  void place(const unsigned short* idx, const long long* off, int nc, int rows) {
+    at_.assign(size_t(rows) * kSlice, -1);
+    for (int l0 = 0; l0 < nc; l0 += 8) {
+      const int nl = std::min(8, nc - l0);
+      // each lane's entries by class (stable)
+      int first[8][9], left[8][8], total[8];
+      sorted_.resize(size_t(off[l0 + nl] - off[l0]));
+      for (int l = 0; l < nl; ++l) {
+        int n[8] = {0};
+        const long long b = off[l0 + l], e = off[l0 + l + 1];
+        for (long long k = b; k < e; ++k) ++n[idx[k] & 7];
+        first[l][0] = int(b - off[l0]);
+        for (int c = 0; c < 8; ++c) {
+          first[l][c + 1] = first[l][c] + n[c];
+          left[l][c] = n[c];
+        }
+        int fill[8];
+        for (int c = 0; c < 8; ++c) fill[c] = first[l][c];
+        for (long long k = b; k < e; ++k) sorted_[size_t(fill[idx[k] & 7]++)] = k;
+        total[l] = int(e - b);
+      }
+      for (int r = 0; r < rows; ++r) {
+        unsigned used = 0;
+        for (int x = 0; x < nl; ++x) {
+          const int l = (x + r) % nl;
+          if (total[l] <= r) continue;
+          int best = -1, any = -1;
+          for (int c = 0; c < 8; ++c) {
+            if (left[l][c] == 0) continue;
+            if (any < 0 || left[l][c] > left[l][any]) any = c;
+            if (!((used >> c) & 1u) && (best < 0 || left[l][c] > left[l][best])) best = c;
+          }
+          const int c = best >= 0 ? best : any;
+          used |= 1u << c;
+          at_[size_t(r) * kSlice + l0 + l] = sorted_[size_t(first[l][c] + --left[l][c])];
+        }
+      }
+    }
+  }
+  long long at(int r, int l) const { return at_[size_t(r) * kSlice + l]; }
+
+ private:
+  std::vector<long long> at_, sorted_;
+};
+}  // namespace
+
 extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** out) {
   if (!d || !out) return fail(CGX_E_ARG, "cgx_mesh_create: null argument");
   *out = nullptr;
@@ -3258,19 +3388,39 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
       }
       std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return key[a] < key[b]; });
     }
+    // ---- inside each work item cells are ordered by their extended faces,
+    // most first (stable), so that the rows of a slice have few empty lanes
+    const int icells = item_cells(N);
+    {
+      int bad_ef = 0;
+#pragma omp parallel for schedule(static) reduction(| : bad_ef)
+      for (int f = 0; f < nef; ++f) {
+        const int a = d->cvoef[2 * size_t(f)], b = d->cvoef[2 * size_t(f) + 1];
+        bad_ef |= (a < 0 || a >= N || b < 0 || b >= ncv_g2);
+      }
+      if (bad_ef) return bail(fail(CGX_E_ARG, "cvoef out of range"));
+      std::vector<int> nfaces(N, 0);
+#pragma omp parallel for schedule(static)
+      for (int f = 0; f < nef; ++f) {
+        const int a = d->cvoef[2 * size_t(f)], b = d->cvoef[2 * size_t(f) + 1];
+#pragma omp atomic
+        ++nfaces[a];
+        if (b < N) {
+#pragma omp atomic
+          ++nfaces[b];
+        }
+      }
+#pragma omp parallel for schedule(static)
+      for (int c0 = 0; c0 < N; c0 += icells)
+        std::stable_sort(perm.begin() + c0, perm.begin() + std::min(c0 + icells, N),
+                         [&](int a, int b) { return nfaces[a] > nfaces[b]; });
+    }
     std::vector<int> iperm(N);
     for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
     auto nw = [&](int idx) { return iperm[owner(idx)]; };
 
     PT.mark("renumbering");
     // ---- match compact faces to extended faces (FlowSolver.hpp:1833-1900)
-    int bad_ef = 0;
-#pragma omp parallel for schedule(static) reduction(| : bad_ef)
-    for (int f = 0; f < nef; ++f) {
-      const int a = d->cvoef[2 * size_t(f)], b = d->cvoef[2 * size_t(f) + 1];
-      bad_ef |= (a < 0 || a >= N || b < 0 || b >= ncv_g2);
-    }
-    if (bad_ef) return bail(fail(CGX_E_ARG, "cvoef out of range"));
     std::vector<int> ef_i(N + 1, 0);
 #pragma omp parallel for schedule(static)
     for (int f = 0; f < nef; ++f) {
@@ -3297,130 +3447,60 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
         if (d->cvoef[2 * size_t(ef_v[k]) + 1] == b) return ef_v[k];
       return -1;
     };
-    std::vector<int> cf_of_ef(nef, -1);
-    std::vector<signed char> cf_rev(nef, 0);
+    uvec<int> cf_of_ef(nef);
+    uvec<CFRec> cfr(std::max(nfa, 1));  // per compact face, its normal along the extended face
     {
-      uvec<int> ef_of_fa(nfa);
-      uvec<signed char> rev_of_fa(nfa);
-      int bad_fa = 0, unmatched = 0;
-#pragma omp parallel for schedule(static) reduction(| : bad_fa, unmatched)
+#pragma omp parallel for schedule(static)
+      for (int f = 0; f < nef; ++f) cf_of_ef[f] = -1;
+      int bad_fa = 0, unmatched = 0, doubled = 0;
+#pragma omp parallel for schedule(static) reduction(| : bad_fa, unmatched, doubled)
       for (int fa = 0; fa < nfa; ++fa) {
         const int a = d->cvofa[2 * size_t(fa)], b = d->cvofa[2 * size_t(fa) + 1];
-        int f = -1;
-        signed char rev = 0;
         if (a < 0 || a >= N || b < 0 || b >= ncv_g2) {
           bad_fa = 1;
-        } else {
-          f = find_ef(a, b);
-          if (f < 0) {
-            f = find_ef(b, a);
-            rev = 1;
-          }
-          unmatched |= (f < 0);
+          continue;
         }
-        ef_of_fa[fa] = f;
-        rev_of_fa[fa] = rev;
-      }
-      if (bad_fa) return bail(fail(CGX_E_ARG, "cvofa out of range"));
-      if (unmatched) return bail(fail(CGX_E_ARG, "compact face without extended face"));
-      for (int fa = 0; fa < nfa; ++fa) {
-        const int f = ef_of_fa[fa];
-        if (cf_of_ef[f] >= 0) return bail(fail(CGX_E_ARG, "two compact faces on one extended face"));
-        cf_of_ef[f] = fa;
-        cf_rev[f] = rev_of_fa[fa];
-      }
-    }
-    PT.mark("compact/extended match");
-    // ---- face numbering: compact faces first, each group ordered by the
-    // first cell (new numbering) that reads the face, then by input face
-    // order: a stable counting sort on the bucket 2*first + (extended only),
-    // in parallel over fixed chunks of faces (per-chunk bucket counts), so
-    // the numbering does not depend on the thread count
-    uvec<int> fnew(nef);
-    {
-      uvec<int> fbucket(nef);
-#pragma omp parallel for schedule(static)
-      for (int f = 0; f < nef; ++f) {
-        const int a = d->cvoef[2 * size_t(f)], b = d->cvoef[2 * size_t(f) + 1];
-        const int na = iperm[a];
-        const int first = (b < N) ? std::min(na, iperm[b]) : na;
-        fbucket[f] = (cf_of_ef[f] >= 0) ? first : N + first;
-      }
-      const size_t NB = 2 * size_t(N);
-      const int nchunk = int(std::min<long long>(16, std::max<long long>(1, nef / 65536)));
-      auto chunk_lo = [&](int c) { return int((long long)nef * c / nchunk); };
-      uvec<int> ccnt(size_t(nchunk) * NB);
-#pragma omp parallel for schedule(static, 1)
-      for (int c = 0; c < nchunk; ++c) {
-        int* cc = ccnt.data() + size_t(c) * NB;
-        std::fill(cc, cc + NB, 0);
-        for (int f = chunk_lo(c); f < chunk_lo(c + 1); ++f) ++cc[fbucket[f]];
-      }
-      // per bucket: the buckets before it, then the chunks before this one
-      std::vector<long long> btot(NB + 1, 0);
-#pragma omp parallel for schedule(static)
-      for (long long k = 0; k < (long long)NB; ++k) {
-        long long t = 0;
-        for (int c = 0; c < nchunk; ++c) t += ccnt[size_t(c) * NB + k];
-        btot[k + 1] = t;
-      }
-      for (size_t k = 0; k < NB; ++k) btot[k + 1] += btot[k];
-#pragma omp parallel for schedule(static)
-      for (long long k = 0; k < (long long)NB; ++k) {
-        long long run = btot[k];
-        for (int c = 0; c < nchunk; ++c) {
-          const int n = ccnt[size_t(c) * NB + k];
-          ccnt[size_t(c) * NB + k] = int(run);
-          run += n;
+        int f = find_ef(a, b);
+        const bool rev = f < 0;
+        if (rev) f = find_ef(b, a);
+        if (f < 0) {
+          unmatched = 1;
+          continue;
         }
-      }
-#pragma omp parallel for schedule(static, 1)
-      for (int c = 0; c < nchunk; ++c) {
-        int* cc = ccnt.data() + size_t(c) * NB;
-        for (int f = chunk_lo(c); f < chunk_lo(c + 1); ++f) fnew[f] = cc[fbucket[f]]++;
-      }
-    }
-    int ncf = 0;
-#pragma omp parallel for schedule(static) reduction(+ : ncf)
-    for (int f = 0; f < nef; ++f) ncf += (cf_of_ef[f] >= 0);
-    uvec<EFRec> efr(nef);
-    uvec<CFRec> cfr(std::max(ncf, 1));
-#pragma omp parallel for schedule(static)
-    for (int f = 0; f < nef; ++f) {
-      EFRec& r = efr[fnew[f]];
-      for (int k = 0; k < 3; ++k) {
-        r.n[k] = d->n_ef[3 * size_t(f) + k];
-        r.c[k] = d->c_ef[3 * size_t(f) + k];
-      }
-      for (int k = 0; k < 3; ++k) r.c[k] *= 0.5;  // FlowSolver.hpp:2256-2259
-      const int fa = cf_of_ef[f];
-      if (fa >= 0) {
+        int was;
+#pragma omp atomic capture
+        {
+          was = cf_of_ef[f];
+          cf_of_ef[f] = fa;
+        }
+        doubled |= (was >= 0);
         // FaCompact (FlowSolver.hpp:1871-1884): unit normal along the
         // extended face, area, area_over_delta; delta = area/area_over_delta
         // as calcInternalCompactFluxNewGrad forms it
-        CFRec& c = cfr[fnew[f]];
+        CFRec& c = cfr[fa];
         const double* n = d->n_fa + 3 * size_t(fa);
         const double area = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
         const double inv_area = 1.0 / area;
-        for (int k = 0; k < 3; ++k) c.un[k] = cf_rev[f] ? -n[k] * inv_area : n[k] * inv_area;
+        for (int k = 0; k < 3; ++k) c.un[k] = rev ? -n[k] * inv_area : n[k] * inv_area;
         c.area = area;
         c.aod = d->area_over_delta_fa[fa];
         c.delta = area / c.aod;
       }
+      if (bad_fa) return bail(fail(CGX_E_ARG, "cvofa out of range"));
+      if (unmatched) return bail(fail(CGX_E_ARG, "compact face without extended face"));
+      if (doubled) return bail(fail(CGX_E_ARG, "two compact faces on one extended face"));
     }
-    PT.mark("face numbering");
+    PT.mark("compact/extended match");
     // ---- directed entries per cell (new numbering): CSR, each cell's entries
-    // by face id, so compact faces (ids < ncf) come first.  A stable counting
-    // sort of the entries, taken in face-id order, by their cell: per chunk of
-    // face ids a count per cell, the chunks' offsets within each cell, then
-    // the chunks scatter in order.  The result does not depend on the chunking.
-    std::vector<int> deg(N, 0), ncomp(N, 0);
-    std::vector<long long> cell_off(N + 1, 0);
+    // by face, kCompactBit in e_nbr marking the compact ones.  A stable counting
+    // sort of the entries, taken in face order, by their cell: per chunk of
+    // faces a count per cell, the chunks' offsets within each cell, then the
+    // chunks scatter in order.  The result does not depend on the chunking.
+    std::vector<int> deg(N, 0);
+    std::vector<long long> cell_off(N + 1, 0), qoff(N + 1, 0);
     uvec<int> e_nbr, e_fid;
+    uvec<unsigned short> q_ent;  // compact entries: position in the cell's list
     {
-      uvec<int> ef_of_fid(nef);
-#pragma omp parallel for schedule(static)
-      for (int f = 0; f < nef; ++f) ef_of_fid[fnew[f]] = f;
       const int nchunk = std::max(1, std::min(omp_get_max_threads(), 32));
       auto chunk_lo = [&](int c) { return int((long long)nef * c / nchunk); };
       uvec<int> cnt(size_t(nchunk) * N);
@@ -3428,15 +3508,15 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
       for (int c = 0; c < nchunk; ++c) {
         int* cc = cnt.data() + size_t(c) * N;
         std::fill(cc, cc + N, 0);
-        for (int fid = chunk_lo(c); fid < chunk_lo(c + 1); ++fid) {
-          const int f = ef_of_fid[fid];
+        for (int f = chunk_lo(c); f < chunk_lo(c + 1); ++f) {
           const int b = d->cvoef[2 * size_t(f) + 1];
           ++cc[iperm[d->cvoef[2 * size_t(f)]]];
           if (b < N) ++cc[iperm[b]];
         }
       }
       // per cell: the chunks' counts become their offsets within the cell
-#pragma omp parallel for schedule(static)
+      int too_many = 0;
+#pragma omp parallel for schedule(static) reduction(| : too_many)
       for (int i = 0; i < N; ++i) {
         int run = 0;
         for (int c = 0; c < nchunk; ++c) {
@@ -3446,33 +3526,43 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
           run += n;
         }
         deg[i] = run;
+        too_many |= (run > 0xffff);
       }
+      if (too_many) return bail(fail(CGX_E_ARG, "a cell has more than 65535 faces"));
       for (int i = 0; i < N; ++i) cell_off[i + 1] = cell_off[i] + deg[i];
       e_nbr.resize(cell_off[N]);
       e_fid.resize(cell_off[N]);
 #pragma omp parallel for schedule(static, 1)
       for (int c = 0; c < nchunk; ++c) {
         int* cc = cnt.data() + size_t(c) * N;
-        for (int fid = chunk_lo(c); fid < chunk_lo(c + 1); ++fid) {
-          const int f = ef_of_fid[fid];
+        for (int f = chunk_lo(c); f < chunk_lo(c + 1); ++f) {
           const int a = d->cvoef[2 * size_t(f)], b = d->cvoef[2 * size_t(f) + 1];
           const int na = iperm[a];
           const int nb = nw(b);
+          const int compact = (cf_of_ef[f] >= 0) ? kCompactBit : 0;
           const long long ka = cell_off[na] + cc[na]++;
-          e_nbr[ka] = nb;
-          e_fid[ka] = fid;
+          e_nbr[ka] = nb | compact;
+          e_fid[ka] = f;
           if (b < N) {
             const long long kb = cell_off[nb] + cc[nb]++;
-            e_nbr[kb] = na;
-            e_fid[kb] = fid | kRevBit;
+            e_nbr[kb] = na | compact;
+            e_fid[kb] = f | kRevBit;
           }
         }
       }
 #pragma omp parallel for schedule(static)
       for (int i = 0; i < N; ++i) {
         int n = 0;
-        for (long long k = cell_off[i]; k < cell_off[i + 1] && (e_fid[k] & kFidMask) < ncf; ++k) ++n;
-        ncomp[i] = n;
+        for (long long k = cell_off[i]; k < cell_off[i + 1]; ++k) n += (e_nbr[k] < 0);
+        deg[i] = n;
+      }
+      for (int i = 0; i < N; ++i) qoff[i + 1] = qoff[i] + deg[i];
+      q_ent.resize(std::max(qoff[N], 1LL));
+#pragma omp parallel for schedule(static)
+      for (int i = 0; i < N; ++i) {
+        long long q = qoff[i];
+        for (long long k = cell_off[i]; k < cell_off[i + 1]; ++k)
+          if (e_nbr[k] < 0) q_ent[q++] = (unsigned short)(k - cell_off[i]);
       }
     }
     PT.mark("entry CSR");
@@ -3485,16 +3575,12 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
       coff[i + 1] = coff[i] + cd;
     }
     uvec<int> c_nbr(coff[N]);
-    uvec<double> gx(coff[N]), gy(coff[N]), gz(coff[N]);
 #pragma omp parallel for schedule(static)
     for (int i = 0; i < N; ++i) {
       const int coc0 = d->cvocv_i[perm[i]] + 1;
       for (long long k = coff[i]; k < coff[i + 1]; ++k) {
         const int coc = coc0 + int(k - coff[i]);
         c_nbr[k] = nw(d->cvocv_v[coc]);
-        gx[k] = d->cvocv_grad_coeff[3 * size_t(coc)];
-        gy[k] = d->cvocv_grad_coeff[3 * size_t(coc) + 1];
-        gz[k] = d->cvocv_grad_coeff[3 * size_t(coc) + 2];
       }
     }
     PT.mark("gradient CSR");
@@ -3549,13 +3635,11 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     std::vector<int> hcell, chcell;
     // (every entry of these is written below)
     uvec<unsigned short> lidx(std::max(cell_off[N], 1LL)), clidx;
-    std::vector<long long> qoff(N + 1, 0);
-    for (int i = 0; i < N; ++i) qoff[i + 1] = qoff[i] + ncomp[i];
     clidx.resize(std::max(qoff[N], 1LL));
     uvec<unsigned short> cglidx(std::max(coff[N], 1LL));
     int max_u = 0, max_cu = 0;
     {
-      // Base items of kItemCells cells are independent: each is built in
+      // Base items of icells cells are independent: each is built in
       // parallel (and split in halves, first half first, while its unions
       // exceed the staging budget), then the items are concatenated in cell
       // order.  The result does not depend on the thread count.
@@ -3563,7 +3647,7 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
         int c0, nc;
         std::vector<int> halo, chalo;  // ascending
       };
-      const int nbase = (N + kItemCells - 1) / kItemCells;
+      const int nbase = (N + icells - 1) / icells;
       std::vector<std::vector<SubItem>> sub(nbase);
       int too_big = 0;
 #pragma omp parallel
@@ -3583,13 +3667,13 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
           chalo.clear();
           for (int i = c0; i < c0 + nc; ++i) {
             for (long long k = cell_off[i]; k < cell_off[i + 1]; ++k) {
-              const int j = e_nbr[k];
+              const int j = e_nbr[k] & kFidMask;
               if (j >= c0 && j < c0 + nc) continue;
               if (seen_h[j] != tag) {
                 seen_h[j] = tag;
                 halo.push_back(j);
               }
-              if (k < cell_off[i] + ncomp[i] && seen_c[j] != tag) {
+              if (e_nbr[k] < 0 && seen_c[j] != tag) {
                 seen_c[j] = tag;
                 chalo.push_back(j);
               }
@@ -3609,7 +3693,7 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
         };
 #pragma omp for schedule(dynamic, 16) reduction(| : too_big)
         for (int bi = 0; bi < nbase; ++bi) {
-          std::vector<std::pair<int, int>> todo{{bi * kItemCells, std::min(kItemCells, N - bi * kItemCells)}};
+          std::vector<std::pair<int, int>> todo{{bi * icells, std::min(icells, N - bi * icells)}};
           while (!todo.empty()) {
             const auto [c0, nc] = todo.back();
             todo.pop_back();
@@ -3617,7 +3701,9 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
             unions(c0, nc, si.halo, si.chalo);
             const int nu = nc + int(si.halo.size()), ncu = nc + int(si.chalo.size());
             if ((nu > kMaxUnionExt || ncu > kMaxUnionComp) && nc > 1) {
-              const int h1 = nc / 2;  // split, first half processed first
+              // split, first half processed first; at a slice's edge while
+              // there is one inside
+              const int h1 = (nc > kSlice) ? std::max(kSlice, nc / 2 / kSlice * kSlice) : nc / 2;
               todo.push_back({c0 + h1, nc - h1});
               todo.push_back({c0, h1});
               continue;
@@ -3627,12 +3713,12 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
               break;
             }
             for (int i = c0; i < c0 + nc; ++i) {
+              long long q = qoff[i];
               for (long long k = cell_off[i]; k < cell_off[i + 1]; ++k) {
-                const int j = e_nbr[k];
+                const int j = e_nbr[k] & kFidMask;
                 const bool in = j >= c0 && j < c0 + nc;
                 lidx[k] = in ? (unsigned short)(j - c0) : loc_h[j];
-                const long long t = k - cell_off[i];
-                if (t < ncomp[i]) clidx[qoff[i] + t] = in ? (unsigned short)(j - c0) : loc_c[j];
+                if (e_nbr[k] < 0) clidx[q++] = in ? (unsigned short)(j - c0) : loc_c[j];
               }
               for (long long k = coff[i]; k < coff[i + 1]; ++k) {
                 const int j = c_nbr[k];
@@ -3675,19 +3761,98 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
       }
       if (bad_local) return bail(fail(CGX_E_ARG, "internal: local index outside its work item's union"));
     }
+    PT.mark("items and halos");
+    // ---- rows of the slices: counts, row offsets, then each slice's entries
+    // placed row by row in the order that place_entries chooses
+    const int nslice = (N + kSlice - 1) / kSlice;
+    std::vector<ushort4> cnt(N);
+    std::vector<int> erow(nslice + 1, 0), qrow(nslice + 1, 0), grow(nslice + 1, 0);
+    {
+      int too_many = 0;
+#pragma omp parallel for schedule(static) reduction(| : too_many)
+      for (int t = 0; t < nslice; ++t) {
+        int me = 0, mq = 0, mg = 0;
+        for (int i = t * kSlice; i < std::min(N, (t + 1) * kSlice); ++i) {
+          const int ne = int(cell_off[i + 1] - cell_off[i]), nq = int(qoff[i + 1] - qoff[i]);
+          const long long ng = coff[i + 1] - coff[i];
+          too_many |= (ng > 0xffff);
+          cnt[i] = make_ushort4((unsigned short)ne, (unsigned short)nq, (unsigned short)ng, 0);
+          me = std::max(me, ne);
+          mq = std::max(mq, nq);
+          mg = std::max(mg, int(ng));
+        }
+        erow[t + 1] = me;
+        qrow[t + 1] = mq;
+        grow[t + 1] = mg;
+      }
+      if (too_many) return bail(fail(CGX_E_ARG, "a cell has more than 65535 faces"));
+      for (int t = 0; t < nslice; ++t) {
+        erow[t + 1] += erow[t];
+        qrow[t + 1] += qrow[t];
+        grow[t + 1] += grow[t];
+      }
+    }
+    const long long E = (long long)erow[nslice] * kSlice, Qn = (long long)qrow[nslice] * kSlice;
+    const long long Cn = (long long)grow[nslice] * kSlice;
+    uvec<unsigned short> s_lidx(std::max(E, 1LL)), s_clidx(std::max(Qn, 1LL)), s_qmap(std::max(Qn, 1LL));
+    uvec<unsigned short> s_cglidx(std::max(Cn, 1LL));
+    uvec<int> s_fid(std::max(E, 1LL)), s_qfid(std::max(Qn, 1LL));
+    uvec<double> s_gc(3 * size_t(std::max(Cn, 1LL)));
+#pragma omp parallel
+    {
+      std::vector<unsigned short> ext_row;  // a cell's entry -> its extended row
+      RowOrder ord;
+#pragma omp for schedule(dynamic, 64)
+      for (int t = 0; t < nslice; ++t) {
+        const int c0 = t * kSlice, nc = std::min(kSlice, N - c0);
+        const long long k0 = cell_off[c0];
+        ext_row.resize(size_t(cell_off[c0 + nc] - k0));
+        ord.place(lidx.data(), cell_off.data() + c0, nc, erow[t + 1] - erow[t]);
+        for (int r = 0; r < erow[t + 1] - erow[t]; ++r)
+          for (int l = 0; l < kSlice; ++l) {
+            const size_t o = (size_t(erow[t]) + r) * kSlice + l;
+            const long long k = ord.at(r, l);
+            if (k >= 0) ext_row[size_t(k - k0)] = (unsigned short)r;
+            s_lidx[o] = k >= 0 ? lidx[k] : 0;
+            s_fid[o] = k >= 0 ? e_fid[k] : kNoFace;
+          }
+        ord.place(clidx.data(), qoff.data() + c0, nc, qrow[t + 1] - qrow[t]);
+        for (int r = 0; r < qrow[t + 1] - qrow[t]; ++r)
+          for (int l = 0; l < kSlice; ++l) {
+            const size_t o = (size_t(qrow[t]) + r) * kSlice + l;
+            const long long q = ord.at(r, l);
+            const long long k = q >= 0 ? cell_off[c0 + l] + q_ent[q] : -1;
+            s_clidx[o] = q >= 0 ? clidx[q] : 0;
+            s_qmap[o] = q >= 0 ? ext_row[size_t(k - k0)] : 0;
+            s_qfid[o] = q >= 0 ? (cf_of_ef[e_fid[k] & kFidMask] | (e_fid[k] & kRevBit)) : kNoFace;
+          }
+        ord.place(cglidx.data(), coff.data() + c0, nc, grow[t + 1] - grow[t]);
+        for (int r = 0; r < grow[t + 1] - grow[t]; ++r)
+          for (int l = 0; l < kSlice; ++l) {
+            const size_t o = size_t(grow[t]) + r;
+            const long long k = ord.at(r, l);
+            s_cglidx[o * kSlice + l] = k >= 0 ? cglidx[k] : 0;
+            const double* c = k >= 0 ? d->cvocv_grad_coeff +
+                                           3 * (size_t(d->cvocv_i[perm[c0 + l]]) + 1 + size_t(k - coff[c0 + l]))
+                                     : nullptr;
+            for (int x = 0; x < 3; ++x) s_gc[(3 * o + x) * kSlice + l] = c ? c[x] : 0.0;
+          }
+      }
+    }
+    PT.mark("rows");
+    std::vector<int> item_of(N);
+    for (const Item& it : items) std::fill(item_of.begin() + it.cell0, item_of.begin() + it.cell0 + it.ncell, it.idx);
     if (hcell.empty()) hcell.push_back(0);
     if (chcell.empty()) chcell.push_back(0);
-    PT.mark("items and halos");
     // ---- upload; the per-face records are expanded on the device into the
-    // per-entry planes and then released
+    // rows and then released
     size_t* acc = &M->bytes;
     int rc;
-    const long long E = cell_off[N];
-    const long long Qn = qoff[N];
-    long long *d_off, *d_qoff, *d_coff;
-    int *d_nbr, *d_cnbr, *d_hcell, *d_chcell;
-    unsigned short *d_lidx, *d_clidx, *d_cglidx;
-    double *d_gx, *d_gy, *d_gz, *d_vol, *d_ivol, *d_en, *d_qg;
+    int *d_erow, *d_qrow, *d_grow;
+    ushort4* d_cnt;
+    int *d_item_of, *d_hcell, *d_chcell;
+    unsigned short *d_lidx, *d_clidx, *d_qmap, *d_cglidx;
+    double *d_gc, *d_vol, *d_ivol, *d_en, *d_qg;
     double4* d_cc;
     Item* d_items;
     cgx_staging::Staging stage(0);
@@ -3703,17 +3868,16 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     UP(d_items, items);
     UP(d_hcell, hcell);
     UP(d_chcell, chcell);
-    UP(d_off, cell_off);
-    UP(d_qoff, qoff);
-    UP(d_nbr, e_nbr);
-    UP(d_lidx, lidx);
-    UP(d_clidx, clidx);
-    UP(d_cglidx, cglidx);
-    UP(d_coff, coff);
-    UP(d_cnbr, c_nbr);
-    UP(d_gx, gx);
-    UP(d_gy, gy);
-    UP(d_gz, gz);
+    UP(d_erow, erow);
+    UP(d_qrow, qrow);
+    UP(d_grow, grow);
+    UP(d_cnt, cnt);
+    UP(d_item_of, item_of);
+    UP(d_lidx, s_lidx);
+    UP(d_clidx, s_clidx);
+    UP(d_qmap, s_qmap);
+    UP(d_cglidx, s_cglidx);
+    UP(d_gc, s_gc);
     UP(d_vol, vol);
     UP(d_ivol, inv_vol);
     UP(d_cc, cc);
@@ -3733,27 +3897,27 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     if ((rc = dalloc(&d_qg, 6 * size_t(std::max(Qn, 1LL)), acc))) return bail(rc);
     M->allocs.push_back(d_qg);
     {
-      std::vector<long long> eofq(std::max(Qn, 1LL), 0);
-      for (int i = 0; i < N; ++i)
-        for (int t = 0; t < ncomp[i]; ++t) eofq[qoff[i] + t] = cell_off[i] + t;
-      int* t_fid = nullptr;
-      EFRec* t_ef = nullptr;
+      int *t_fid = nullptr, *t_qfid = nullptr;
+      double *t_n = nullptr, *t_c = nullptr;
       CFRec* t_cf = nullptr;
-      long long* t_eofq = nullptr;
       auto free_tmp = [&] {
         cudaFree(t_fid);
-        cudaFree(t_ef);
+        cudaFree(t_qfid);
+        cudaFree(t_n);
+        cudaFree(t_c);
         cudaFree(t_cf);
-        cudaFree(t_eofq);
       };
-      if ((rc = dupload(&t_fid, e_fid, nullptr, &stage)) || (rc = dupload(&t_ef, efr, nullptr, &stage)) ||
-          (rc = dupload(&t_cf, cfr, nullptr, &stage)) || (rc = dupload(&t_eofq, eofq, nullptr, &stage))) {
+      if ((rc = dupload(&t_fid, s_fid, nullptr, &stage)) || (rc = dupload(&t_qfid, s_qfid, nullptr, &stage)) ||
+          (rc = dupload(&t_n, d->n_ef, 3 * size_t(nef), &stage)) || (rc = dupload(&t_c, d->c_ef, 3 * size_t(nef), &stage)) ||
+          (rc = dupload(&t_cf, cfr, nullptr, &stage))) {
         free_tmp();
         return bail(rc);
       }
       const long long nmax = std::max(E, Qn);
       if (nmax > 0)
-        k_expand_entries<<<int((nmax + 255) / 256), 256>>>(E, Qn, t_fid, t_ef, t_cf, t_eofq, d_en, d_qg);
+        k_expand_entries<<<int((nmax + 255) / 256), 256>>>(E, Qn, t_fid, t_qfid, t_n, t_c, t_cf,
+                                                                reinterpret_cast<double2*>(d_en),
+                                                                reinterpret_cast<double2*>(d_qg));
       const cudaError_t ke = cudaGetLastError();
       const cudaError_t se = cudaDeviceSynchronize();
       free_tmp();
@@ -3766,23 +3930,22 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     md.N = N;
     md.nitems = int(items.size());
     md.E = E;
-    md.Q = Qn;
     md.items = d_items;
     md.hcell = d_hcell;
     md.chcell = d_chcell;
-    md.off = d_off;
-    md.qoff = d_qoff;
-    md.nbr = d_nbr;
+    md.erow = d_erow;
+    md.qrow = d_qrow;
+    md.grow = d_grow;
+    md.cnt = d_cnt;
+    md.item_of = d_item_of;
+    md.nbr = nullptr;
     md.lidx = d_lidx;
     md.clidx = d_clidx;
+    md.qmap = d_qmap;
     md.cglidx = d_cglidx;
     md.en = d_en;
     md.qg = d_qg;
-    md.coff = d_coff;
-    md.cnbr = d_cnbr;
-    md.gcx = d_gx;
-    md.gcy = d_gy;
-    md.gcz = d_gz;
+    md.gc = d_gc;
     md.vol = d_vol;
     md.inv_vol = d_ivol;
     md.cc = d_cc;
@@ -3796,11 +3959,12 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     md.bf_zone = d_bfz;
     md.en32 = nullptr;
     md.qg32 = nullptr;
-    md.gcx32 = md.gcy32 = md.gcz32 = nullptr;
+    md.gc32 = nullptr;
     M->items = items;
     M->max_union = max_u;
     M->max_cunion = max_cu;
-    M->nc_dir = coff[N];
+    M->nq = Qn;
+    M->nc = Cn;
     long long n_ef_dir = cell_off[N], n_cf_dir = qoff[N];
     M->stats.ncv = N;
     M->stats.n_ef_dir = n_ef_dir;
@@ -3899,30 +4063,23 @@ extern "C" int cgx_solver_create(cgx_mesh* m, const cgx_params* p, cgx_precision
     AL(sd.VF, N);
     AL(sd.QF, N);
     if (!m->have32) {
-      float *en32, *qg32, *gx32, *gy32, *gz32;
+      float *en32, *qg32, *gc32;
       size_t* mb = &m->bytes;
       const MeshDev& md = m->md;
       if ((rc = dalloc(&en32, 6 * size_t(std::max(md.E, 1LL)), mb))) return bail(rc);
       m->allocs.push_back(en32);
-      if ((rc = dalloc(&qg32, 6 * size_t(std::max(md.Q, 1LL)), mb))) return bail(rc);
+      if ((rc = dalloc(&qg32, 6 * size_t(std::max(m->nq, 1LL)), mb))) return bail(rc);
       m->allocs.push_back(qg32);
-      if ((rc = dalloc(&gx32, m->nc_dir, mb))) return bail(rc);
-      m->allocs.push_back(gx32);
-      if ((rc = dalloc(&gy32, m->nc_dir, mb))) return bail(rc);
-      m->allocs.push_back(gy32);
-      if ((rc = dalloc(&gz32, m->nc_dir, mb))) return bail(rc);
-      m->allocs.push_back(gz32);
-      const long long nmax = std::max(6 * md.E, std::max(6 * md.Q, m->nc_dir));
-      k_geom32<<<int((nmax + 255) / 256), 256, 0, s->stream>>>(6 * md.E, 6 * md.Q, m->nc_dir, md.en, md.qg,
-                                                               md.gcx, md.gcy, md.gcz, en32, qg32, gx32,
-                                                               gy32, gz32);
+      if ((rc = dalloc(&gc32, 3 * size_t(std::max(m->nc, 1LL)), mb))) return bail(rc);
+      m->allocs.push_back(gc32);
+      const long long nmax = std::max(6 * md.E, std::max(6 * m->nq, 3 * m->nc));
+      k_geom32<<<int((nmax + 255) / 256), 256, 0, s->stream>>>(6 * md.E, 6 * m->nq, 3 * m->nc, md.en, md.qg, md.gc,
+                                                               en32, qg32, gc32);
       if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s->stream) != cudaSuccess)
         return bail(fail(CGX_E_CUDA, "FP32 geometry conversion failed"));
       m->md.en32 = en32;
       m->md.qg32 = qg32;
-      m->md.gcx32 = gx32;
-      m->md.gcy32 = gy32;
-      m->md.gcz32 = gz32;
+      m->md.gc32 = gc32;
       m->stats.device_bytes = m->bytes;
       m->have32 = true;
     }
@@ -4140,6 +4297,23 @@ extern "C" int cgx_get_state(cgx_solver* s, double* rho, double* u, double* rhoE
   return CGX_OK;
 }
 
+// The extended entries' global neighbours, which only the scalars read, are
+// built when a solver of the mesh first has scalars (4 B per entry).
+static int ensure_nbr(cgx_mesh* m, cudaStream_t stream) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (m->md.nbr) return CGX_OK;
+  int* nbr = nullptr;
+  if (int rc = dalloc(&nbr, size_t(std::max(m->md.E, 1LL)), &m->bytes)) return rc;
+  m->allocs.push_back(nbr);
+  k_fill_nbr<<<m->md.nitems, 128, 0, stream>>>(m->md, nbr);
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
+    return fail(CGX_E_CUDA, "neighbour list of the scalars failed");
+  m->md.nbr = nbr;
+  m->stats.device_bytes = m->bytes;
+  return CGX_OK;
+}
+
 // The scalar arrays (sc, three stages of rhs_sc, per-entry mf) are allocated
 // at the first call with nsc > 0 and kept; a later call with another nsc
 // reallocates them.  Every copy of the case descriptor (host, device table,
@@ -4167,6 +4341,8 @@ extern "C" int cgx_set_scalars(cgx_solver* s, int nsc, const double* sc) {
     if (nsc > 0) {
       const size_t E = size_t(std::max(s->mesh->md.E, 1LL));
       int rc;
+      if ((rc = ensure_nbr(s->mesh, s->stream))) return rc;
+      s->hcase.m.nbr = s->run.dcase.m.nbr = s->mesh->md.nbr;
       if ((rc = dalloc(&sd.sc, size_t(nsc) * N, &s->bytes))) return rc;
       s->allocs.push_back(sd.sc);
       if ((rc = dalloc(&sd.rhs_sc, 3 * size_t(nsc) * N, &s->bytes))) return rc;
@@ -5242,8 +5418,8 @@ size_t solver_bytes(long long N, long long nitems, cgx_precision prec) {
 }
 
 size_t mesh32_bytes(const cgx_mesh* m) {
-  return 6 * size_t(std::max(m->md.E, 1LL)) * sizeof(float) + 6 * size_t(std::max(m->md.Q, 1LL)) * sizeof(float) +
-         size_t(m->nc_dir) * 3 * sizeof(float);
+  return (6 * size_t(std::max(m->md.E, 1LL)) + 6 * size_t(std::max(m->nq, 1LL)) + 3 * size_t(std::max(m->nc, 1LL))) *
+         sizeof(float);
 }
 
 }  // namespace

@@ -4,30 +4,36 @@
 // Data layout in HBM (cells renumbered on a space-filling curve, "new" order):
 //   state    rho[N], u0[N], u1[N], u2[N], rhoE[N]          (SoA, FP64)
 //   rhs      rhs[stage][5][N]                              (SoA, FP64)
-//   LRec[N]  {u0,u1,u2, 1/rho, p, h, rho, sos}  64 B       neighbour gathers
-//   VRec[N]  {mu_total, loc_total, a_sgs, fgr, symh, symp, dudx[9], -}
+//   LRec[N]  {u0,u1,u2, 1/rho, p, rho, h, sos}  64 B       neighbour gathers
+//   VRec[N]  {mu_total, loc_total, a_sgs, fgr, dudx[9], symh, symp, mu_lam}
 //            128 B: lagged properties (per step) and the velocity gradient
 //            (per stage), one 128 B line per neighbour gather
 //   QRec[N]  {log(p/p_ref), p, 1/rho, 1/(R T)}  32 B (Gibbs sensor)
 //   Work items: runs of at most kItemCells consecutive cells.  For each item
 //   the mesh lists its halo, the cells outside the item that its cells'
 //   extended faces reach (hcell) and, separately, those their compact faces
-//   reach (chcell), ascending.  The face-flux kernels copy the packed records
-//   of an item's cells and halo into shared memory once, then every face reads
-//   its neighbour there through a 16-bit local index (the item's own cells
-//   first, then the halo in list order).
-//   Extended-face entries: a CSR over cells (off[N+1]) of directed entries,
-//   one per (cell, face) pair, a cell's compact faces first.  Per entry: the
-//   local index lidx[k], the global neighbour nbr[k] and six FP64 planes
-//   en[d*E + k] {normal along the entry (n[3], negated for the face's second
-//   cell), the halved c vector (c[3])}, streamed contiguously by the cell's G
-//   lanes.
-//   Compact-face entries: the first ncomp(i) = qoff[i+1]-qoff[i] extended
-//   entries of each cell; their local indices in the compact union clidx[q]
-//   and six FP64 planes qg[d*Q + q] {unit normal along the entry (3), area,
-//   area_over_delta, area/area_over_delta} at q = qoff[i] + t.
-//   Gradient coefficients per directed compact entry in a second CSR (coff,
-//   the reference's cvocv order).
+//   reach (chcell), ascending.  The face kernels copy the packed records of an
+//   item's cells and halo into shared memory once, then every face reads its
+//   neighbour there through a 16-bit local index (the item's own cells first,
+//   then the halo in list order).
+//   Slices: 32 consecutive cells [32 s, 32 s + 32), one per lane of a warp.
+//   The directed entries of a slice's cells (one per cell and face) are stored
+//   row by row, row r holding every cell's r-th entry in lane order, so a warp
+//   streams whole rows and each lane sums its own cell: no shuffles, and the
+//   cell's own record stays in registers.  Slice s owns rows [erow[s],
+//   erow[s+1]); a cell has cnt[i].x of them, and inside an item cells are
+//   ordered by that count, so that few lanes of a row are empty.
+//     extended faces: lidx[row][32] local index, en[row][3][32][2] {normal along
+//       the entry (negated for the face's second cell), the halved c vector}
+//     compact faces (rows qrow, count cnt.y): clidx, qmap[row][32] (the cell's
+//       extended row of the same face), qg[row][3][32][2] {unit normal along
+//       the entry, area, area_over_delta, area/area_over_delta}
+//     gradient stencil (rows grow, count cnt.z; the reference's cvocv without
+//       the diagonal): cglidx, gc[row][3][32]
+//   The order of a cell's entries is free.  It is chosen on the host so that
+//   the eight lanes whose 16-byte shared-memory reads are served together find
+//   their neighbours' records in different banks (local indices different
+//   modulo 8) wherever the lists allow it.
 #ifndef CGX_KERNELS_CUH
 #define CGX_KERNELS_CUH
 
@@ -38,26 +44,28 @@ namespace cgx {
 constexpr int kRevBit = 0x80000000;
 constexpr int kMaxScalars = 8;  // transport scalars per cell
 constexpr int kFidMask = 0x7fffffff;
+constexpr int kCompactBit = 0x80000000;
 
 struct alignas(32) LRec {
   double u[3];
   double sp_vol;
   double p;
-  double h;
   double rho;
+  double h;
   double sos;
 };
 
-// per-cell viscous record: lagged properties then dudx[i][j] at g[3*i+j];
-// mu_lam (the laminar viscosity of the wall boundary flux) in the last slot
+// per-cell viscous record: lagged properties and dudx[i][j] at g[3*i+j];
+// mu_lam (the laminar viscosity of the wall boundary flux) in the last slot.
+// Each 32 B sector is written by one kernel only, but for g[8] in the last.
 struct alignas(128) VRec {
   double mu_total;
   double loc_total;
   double a_sgs;
   double fgr;
+  double g[9];
   double symh;
   double symp;
-  double g[9];
   double mu_lam;
 };
 
@@ -68,13 +76,8 @@ struct alignas(32) QRec {
   double ib;  // 1/(R T)
 };
 
-// geometry of one face as built on the host (expanded into the per-entry
-// planes on the device)
-struct alignas(16) EFRec {
-  double n[3];
-  double c[3];  // already halved
-};
-
+// geometry of one compact face as built on the host (expanded into the rows on
+// the device)
 struct alignas(16) CFRec {
   double un[3];  // unit normal along the extended face's orientation
   double area;
@@ -95,9 +98,9 @@ struct alignas(32) LRecF {
 };
 
 struct alignas(64) VRecF {
-  float mu_total, loc_total, a_sgs, fgr, symh, symp;
+  float mu_total, loc_total, a_sgs, fgr;
   float g[9];
-  float mu_lam;
+  float symh, symp, mu_lam;
 };
 
 struct alignas(16) QRecF {
@@ -147,6 +150,9 @@ struct Ctl {
 // A work item: up to kItemCells consecutive cells of one case and where its
 // halo lists start.
 constexpr int kItemCells = 128;
+constexpr int kSlice = 32;  // cells per slice
+// a lane without an entry in a row (the host's face id there)
+constexpr int kNoFace = 0x7fffffff;
 struct alignas(32) Item {
   int c;      // case slot in the table (0 in a mesh's own table)
   int cell0;  // first cell
@@ -161,24 +167,23 @@ struct alignas(32) Item {
 struct MeshDev {
   int N;                        // owned cells
   int nitems;                   // work items (mesh order)
-  long long E;                  // directed extended entries
-  long long Q;                  // directed compact entries
+  long long E;                  // extended rows x 32 (mf's length)
   const Item* items;            // [nitems]
   const int* hcell;             // extended-face halos
   const int* chcell;            // compact-face halos
-  const long long* off;         // [N+1] extended-entry CSR
-  const long long* qoff;        // [N+1] compact-entry CSR
-  const int* nbr;               // [E] neighbour (new numbering, ghosts -> owner)
-  const unsigned short* lidx;   // [E] neighbour in the item's extended union
-  const unsigned short* clidx;  // [Q] neighbour in the item's compact union
-  const double* en;             // [6][E] n (along the entry), c/2
-  const double* qg;             // [6][Q] unit normal, area, aod, delta
-  const long long* coff;        // [N+1] gradient CSR (cvocv without the diagonal)
-  const int* cnbr;              // [C_dir]
-  const unsigned short* cglidx; // [C_dir] neighbour in the item's compact union
-  const double* gcx;            // [C_dir]
-  const double* gcy;
-  const double* gcz;
+  const int* erow;              // [slices+1] rows of extended entries
+  const int* qrow;              // [slices+1] rows of compact entries
+  const int* grow;              // [slices+1] rows of gradient entries
+  const ushort4* cnt;           // [N] the cell's entries: extended, compact, gradient
+  const int* item_of;           // [N] the item that holds the cell
+  const int* nbr;               // [erow][32] neighbour cell (null until a solver has scalars)
+  const unsigned short* lidx;   // [erow][32] neighbour in the item's extended union
+  const unsigned short* clidx;  // [qrow][32] neighbour in the item's compact union
+  const unsigned short* qmap;   // [qrow][32] the entry's row among the cell's extended rows
+  const unsigned short* cglidx; // [grow][32] neighbour in the item's compact union
+  const double* en;             // [erow][3][32][2] n (along the entry), c/2
+  const double* qg;             // [qrow][3][32][2] unit normal, area, aod, delta
+  const double* gc;             // [grow][3][32] gradient coefficients
   const double* vol;
   const double* inv_vol;
   const double4* cc;            // {pow(vol,1/3), pow(vol,2/3), dcmag_hat, sa_to_vol}
@@ -192,11 +197,9 @@ struct MeshDev {
   const double* bf_aod;         // [nbf] area_over_delta_bf
   const int* bf_zone;           // [nbf]
   // FP32 copies for the mixed-precision form (null until a mixed solver exists)
-  const float* en32;            // [6][E]
-  const float* qg32;            // [6][Q]
-  const float* gcx32;
-  const float* gcy32;
-  const float* gcz32;
+  const float* en32;
+  const float* qg32;
+  const float* gc32;
 };
 
 struct StateDev {

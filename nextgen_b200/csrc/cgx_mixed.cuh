@@ -26,40 +26,24 @@ struct FluxF {
 };
 
 // FP32 records in the swizzled shared arrays
-__device__ __forceinline__ void smem_LF(const int4* sm, int j, LRecF& r) {
-  const float4* p = reinterpret_cast<const float4*>(sm);
-  const float4 a = p[swz<2>(j, 0)], b = p[swz<2>(j, 1)];
+__device__ __forceinline__ void smem_LF(const int4* sm, int pl, int j, LRecF& r) {
+  const float4* p = reinterpret_cast<const float4*>(sm) + j;
+  const float4 a = p[0], b = p[pl];
   r.u[0] = a.x; r.u[1] = a.y; r.u[2] = a.z; r.sp_vol = a.w;
   r.pp = b.x; r.hh = b.y; r.rho = b.z; r.sos = b.w;
 }
 
-__device__ __forceinline__ void smem_VF_sum(const int4* sm, int a, int b, VRecF& r) {
-  const float4* p = reinterpret_cast<const float4*>(sm);
-  float4 x = p[swz<4>(a, 0)], y = p[swz<4>(b, 0)];
+__device__ __forceinline__ void smem_VF_sum(const int4* sm, int pl, int a, int b, VRecF& r) {
+  const float4* p = reinterpret_cast<const float4*>(sm) + a;
+  const float4* q = reinterpret_cast<const float4*>(sm) + b;
+  float4 x = p[0], y = q[0];
   r.mu_total = x.x + y.x; r.loc_total = x.y + y.y; r.a_sgs = x.z + y.z; r.fgr = x.w + y.w;
-  x = p[swz<4>(a, 1)]; y = p[swz<4>(b, 1)];
-  r.symh = x.x + y.x; r.symp = x.y + y.y; r.g[0] = x.z + y.z; r.g[1] = x.w + y.w;
-  x = p[swz<4>(a, 2)]; y = p[swz<4>(b, 2)];
-  r.g[2] = x.x + y.x; r.g[3] = x.y + y.y; r.g[4] = x.z + y.z; r.g[5] = x.w + y.w;
-  x = p[swz<4>(a, 3)]; y = p[swz<4>(b, 3)];
-  r.g[6] = x.x + y.x; r.g[7] = x.y + y.y; r.g[8] = x.z + y.z;
-}
-
-// the once-per-step kernel's streams, mixed form
-__device__ __forceinline__ void prefetch_end_f(const MeshDev& m, const Item& it, int sub, int cpr) {
-  const int a = min(sub * cpr, it.ncell), b = min((sub + 1) * cpr, it.ncell);
-  const int t = threadIdx.x;
-  if (a >= b || t >= 6) return;
-  if (t == 0) {
-    const long long k0 = __ldg(m.off + it.cell0 + a), k1 = __ldg(m.off + it.cell0 + b);
-    prefetch_l2(m.lidx + k0, (k1 - k0) * 2);
-    return;
-  }
-  const long long q0 = __ldg(m.qoff + it.cell0 + a), q1 = __ldg(m.qoff + it.cell0 + b);
-  if (t == 5)
-    prefetch_l2(m.clidx + q0, (q1 - q0) * 2);
-  else
-    prefetch_l2(m.qg32 + (t - 1) * m.Q + q0, (q1 - q0) * 4);
+  x = p[pl]; y = q[pl];
+  r.g[0] = x.x + y.x; r.g[1] = x.y + y.y; r.g[2] = x.z + y.z; r.g[3] = x.w + y.w;
+  x = p[2 * pl]; y = q[2 * pl];
+  r.g[4] = x.x + y.x; r.g[5] = x.y + y.y; r.g[6] = x.z + y.z; r.g[7] = x.w + y.w;
+  x = p[3 * pl]; y = q[3 * pl];
+  r.g[8] = x.x + y.x; r.symh = x.y + y.y; r.symp = x.z + y.z;
 }
 
 // ext_flux (cgx.cu) on the FP32 perturbation variables; F[4] excludes the
@@ -167,81 +151,82 @@ __device__ __forceinline__ void compact_flux_add_f(FluxF& F, const float un_[3],
 }
 
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256, 4) k_rhs_ext_f(CASE_ARGS, int stage) {
+__global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 8 : G <= 8 ? 4 : 1) k_rhs_ext_f(CASE_ARGS, int stage) {
   extern __shared__ int4 smem[];
-#define PF_EXTF(it, mm, r) prefetch_round<false>(mm, mm.en32, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_EXTF)
-  stage_records<2>(smem, s.LF, it_, m.hcell + it_.hoff, it_.nh);
-  stage_wait();
-  const long long E = m.E;
+  int4* sL = smem + kWarps<G>() * kSumBytes<double>(5) / 16;
+  STAGED_LOOP_BEGIN(G)
+  Rows<768, float2, 3> rows;
+  ROWS_START(m.erow, x, m.lidx, m.en32, 0)
+  double* const mf = DIRECT ? s.mf : nullptr;
+  const int pl = plane_len(max_u, 2);
+  stage_records<2, 2>(sL, pl, s.LF, it_, m.hcell + it_.hoff, it_.nh);
   const double h_ref = CASE_PH.h_ref;
-  STAGED_ROUNDS_BEGIN(G, PF_EXTF)
-  long long b = 0, e = 0;
+  stage_wait();
+  SLICES_BEGIN(G)
   LRecF Li;
-  if (valid) {
-    b = m.off[i];
-    e = m.off[i + 1];
-    smem_LF(smem, loc_, Li);
-  }
+  if (valid) smem_LF(sL, pl, loc_, Li);
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (long long k = b + lane; k < e; k += G) {
-    const int jl = __ldg(m.lidx + k);
-    const float* g = m.en32 + k;
-    const float n[3] = {__ldg(g), __ldg(g + E), __ldg(g + 2 * E)};
-    const float c[3] = {__ldg(g + 3 * E), __ldg(g + 4 * E), __ldg(g + 5 * E)};
+  size_t k = 0;
+  if (mf && valid) k = (size_t(__ldg(m.erow + slice_)) + part_) * 32 + (threadIdx.x & 31);
+#pragma unroll 1
+  while (rows.left > 0) {
+    float2 g[3];
+    const int jl = rows.next(parts_, g);
     LRecF Lj;
-    smem_LF(smem, jl, Lj);
+    smem_LF(sL, pl, jl, Lj);
+    const float n[3] = {g[0].x, g[0].y, g[1].x}, c[3] = {g[1].y, g[2].x, g[2].y};
     float F[5];
     ext_flux_f(F, n, c, Li, Lj);
-    if (s.mf) s.mf[k] = double(F[0]);  // mass flux for calcRhsScalars
+    if (mf) {  // mass flux for calcRhsScalars
+      mf[k] = double(F[0]);
+      k += 32 * parts_;
+    }
 #pragma unroll
     for (int q = 0; q < 5; ++q) acc[q] -= double(F[q]);
   }
-#pragma unroll
-  for (int c = 0; c < 5; ++c) acc[c] = group_sum<G>(acc[c]);
-  acc[4] += h_ref * acc[0];
-  if (valid) {
+  combine_parts(acc, smem, kSumBytes<double>(5), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
+    acc[4] += h_ref * acc[0];
     double* r = s.rhs + size_t(stage) * 5 * m.N;
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-      if (c % G == lane) r[size_t(c) * m.N + i] = acc[c];
+    for (int c = 0; c < 5; ++c) r[size_t(c) * m.N + i] = acc[c];
   }
-  STAGED_ROUNDS_END
+  if (t_ + spr_ < nsl_) ROWS_START(m.erow, x, m.lidx, m.en32, t_ + spr_)
+  SLICES_END
   STAGED_LOOP_END
-#undef PF_EXTF
 }
 
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256, 3) k_rhs_comp_f(CASE_ARGS, int stage) {
+__global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_rhs_comp_f(CASE_ARGS, int stage) {
   extern __shared__ int4 smem[];
-#define PF_COMPF(it, mm, r) prefetch_round<true>(mm, mm.qg32, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_COMPF)
-  const int nu = it_.ncell + it_.nch;
-  int4* sV = smem + swz_chunks<2>(nu);
-  stage_records<2>(smem, s.LF, it_, m.chcell + it_.choff, it_.nch);
-  stage_records<4>(sV, s.VF, it_, m.chcell + it_.choff, it_.nch);
-  stage_wait();
-  const long long Q = m.Q;
+  int4* sL = smem + kWarps<G>() * kSumBytes<double>(5) / 16;
+  STAGED_LOOP_BEGIN(G)
+  Rows<768, float2, 3> rows;
+  ROWS_START(m.qrow, y, m.clidx, m.qg32, 0)
+  double* const mf = DIRECT ? s.mf : nullptr;
+  const int pl = plane_len(max_cu, 2), pv = plane_len(max_cu, 4);
+  int4* sV = sL + 2 * pl;
+  stage_records<2, 2>(sL, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
+  stage_records<4, 4>(sV, pv, s.VF, it_, m.chcell + it_.choff, it_.nch);
   const double h_ref = CASE_PH.h_ref;
   const float p_ref = float(CASE_PH.p_ref);
-  STAGED_ROUNDS_BEGIN(G, PF_COMPF)
-  long long q0 = 0, q1 = 0;
+  stage_wait();
+  SLICES_BEGIN(G)
   LRecF Li;
-  if (valid) {
-    q0 = m.qoff[i];
-    q1 = m.qoff[i + 1];
-    smem_LF(smem, loc_, Li);
-  }
+  if (valid) smem_LF(sL, pl, loc_, Li);
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (long long q = q0 + lane; q < q1; q += G) {
-    const int jl = __ldg(m.clidx + q);
-    const float* h = m.qg32 + q;
-    const float un[3] = {__ldg(h), __ldg(h + Q), __ldg(h + 2 * Q)};
-    const float area = __ldg(h + 3 * Q), aod = __ldg(h + 4 * Q), delta = __ldg(h + 5 * Q);
+  size_t q = 0;
+  if (mf && valid) q = (size_t(__ldg(m.qrow + slice_)) + part_) * 32 + (threadIdx.x & 31);
+#pragma unroll 1
+  while (rows.left > 0) {
+    float2 h[3];
+    const int jl = rows.next(parts_, h);
+    const float un[3] = {h[0].x, h[0].y, h[1].x};
+    const float area = h[1].y, aod = h[2].x, delta = h[2].y;
     LRecF Lj;
-    smem_LF(smem, jl, Lj);
+    smem_LF(sL, pl, jl, Lj);
     VRecF Vs;
-    smem_VF_sum(sV, loc_, jl, Vs);
+    smem_VF_sum(sV, pv, loc_, jl, Vs);
     float uf[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) uf[d] = 0.5f * (Li.u[d] + Lj.u[d]);
@@ -250,48 +235,50 @@ __global__ void __launch_bounds__(256, 3) k_rhs_comp_f(CASE_ARGS, int stage) {
     FluxF F;
     F.rho = 0.0f; F.ru[0] = F.ru[1] = F.ru[2] = 0.0f; F.rE = 0.0f;
     compact_flux_add_f(F, un, area, aod, delta, Li, Lj, Vs, uf, h_f, p_ref);
-    if (s.mf) s.mf[m.off[i] + (q - q0)] += double(F.rho);  // the closure's mass flux
+    if (mf) {  // the closure's mass flux
+      mf[(size_t(__ldg(m.erow + slice_)) + __ldg(m.qmap + q)) * 32 + (threadIdx.x & 31)] += double(F.rho);
+      q += 32 * parts_;
+    }
     acc[0] -= double(F.rho);
     acc[1] -= double(F.ru[0]);
     acc[2] -= double(F.ru[1]);
     acc[3] -= double(F.ru[2]);
     acc[4] -= double(F.rE);
   }
-#pragma unroll
-  for (int c = 0; c < 5; ++c) acc[c] = group_sum<G>(acc[c]);
-  acc[4] += h_ref * acc[0];
-  if (valid && q1 > q0) {
+  combine_parts(acc, smem, kSumBytes<double>(5), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
+    acc[4] += h_ref * acc[0];
     double* r = s.rhs + size_t(stage) * 5 * m.N;
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-      if (c % G == lane) r[size_t(c) * m.N + i] += acc[c];
+    for (int c = 0; c < 5; ++c) r[size_t(c) * m.N + i] += acc[c];
   }
-  STAGED_ROUNDS_END
+  if (t_ + spr_ < nsl_) ROWS_START(m.qrow, y, m.clidx, m.qg32, t_ + spr_)
+  SLICES_END
   STAGED_LOOP_END
-#undef PF_COMPF
 }
 
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256) k_grad_f(CASE_ARGS) {
+__global__ void __launch_bounds__(kThreads<G>()) k_grad_f(CASE_ARGS) {
   extern __shared__ int4 smem[];
-#define PF_GRADF(it, mm, r) prefetch_grad(mm, mm.gcx32, mm.gcy32, mm.gcz32, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_GRADF)
-  stage_records<1, 2>(smem, s.LF, it_, m.chcell + it_.choff, it_.nch);
+  STAGED_LOOP_BEGIN(G)
+  Rows<384, float, 3> rows;
+  ROWS_START(m.grow, z, m.cglidx, m.gc32, 0)
+  const int pl = plane_len(max_cu, 1);
+  stage_records<1, 2>(smem, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
   const float4* su = reinterpret_cast<const float4*>(smem);
-  STAGED_ROUNDS_BEGIN(G, PF_GRADF)
-  long long b = 0, e = 0;
+  SLICES_BEGIN(G)
   float ui[3] = {0.0f, 0.0f, 0.0f};
   if (valid) {
-    b = m.coff[i];
-    e = m.coff[i + 1];
     const float4 a = su[loc_];
     ui[0] = a.x; ui[1] = a.y; ui[2] = a.z;
   }
   float g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long k = b + lane; k < e; k += G) {
-    const int jl = __ldg(m.cglidx + k);
-    const float cx = __ldg(m.gcx32 + k), cy = __ldg(m.gcy32 + k), cz = __ldg(m.gcz32 + k);
+#pragma unroll 2
+  while (rows.left > 0) {
+    float c[3];
+    const int jl = rows.next(parts_, c);
+    const float cx = c[0], cy = c[1], cz = c[2];
     const float4 ja = su[jl];
     const float du[3] = {ja.x - ui[0], ja.y - ui[1], ja.z - ui[2]};
 #pragma unroll
@@ -301,19 +288,16 @@ __global__ void __launch_bounds__(256) k_grad_f(CASE_ARGS) {
       g[3 * d + 2] += cz * du[d];
     }
   }
-#pragma unroll
-  for (int c = 0; c < 9; ++c) {
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], o);
+  combine_parts(g, smem + pl, kSumBytes<float>(9), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
+    float* P = reinterpret_cast<float*>(s.VF + i);
+    reinterpret_cast<float4*>(P)[1] = make_float4(g[0], g[1], g[2], g[3]);
+    reinterpret_cast<float4*>(P)[2] = make_float4(g[4], g[5], g[6], g[7]);
+    P[12] = g[8];
   }
-  if (valid) {
-#pragma unroll
-    for (int c = 0; c < 9; ++c)
-      if (c % G == lane) s.VF[i].g[c] = g[c];
-  }
-  STAGED_ROUNDS_END
+  if (t_ + spr_ < nsl_) ROWS_START(m.grow, z, m.cglidx, m.gc32, t_ + spr_)
+  SLICES_END
   STAGED_LOOP_END
-#undef PF_GRADF
 }
 
 // cell_props in FP32 (SGS, properties and the sensor function; dt the
@@ -383,99 +367,81 @@ __device__ __forceinline__ int cell_props_f(const Phys& ph, const MeshDev& m, co
   if (ph.diss_mode == CGX_DISS_ALL) fgr = 0.5f;
   float* P = reinterpret_cast<float*>(s.VF + i);
   reinterpret_cast<float4*>(P)[0] = make_float4(mu_lam + mu_sgs, loc_lam + loc_sgs, a_sgs, fgr);
-  reinterpret_cast<float2*>(P)[2] = make_float2(symh, symp);
-  P[15] = mu_lam;
+  reinterpret_cast<float4*>(P)[3] = make_float4(g[8], symh, symp, mu_lam);
   return (rho != rho) || (p != p) || (T != T);
 }
 
 // once per step, mixed form: FP32 SGS/properties/sensor, FP64 CFL sums and
 // reductions (same structure as k_step_end)
 template <int G, bool DIRECT>
-__global__ void __launch_bounds__(256, 3) k_step_end_f(CASE_ARGS, int mode) {
+__global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_step_end_f(CASE_ARGS, int mode) {
   extern __shared__ int4 smem[];
-  __shared__ double sh_cfl[256];
-  __shared__ int sh_nan[256];
-  __shared__ bool am_last;
-#define PF_ENDF(it, mm, r) prefetch_end_f(mm, it, r, 256 / G)
-  STAGED_LOOP_BEGIN(PF_ENDF)
+  int4* sQ = smem + kWarps<G>() * kSumBytes<double>(2) / 16;
+  STAGED_LOOP_BEGIN(G)
+  Rows<768, float2, 2> rows;  // unit normals and areas
+  ROWS_START(m.qrow, y, m.clidx, m.qg32, 0)
+  if (sub_ < spr_ && part_ == 0 && (threadIdx.x & 31) == 0) {
+    const int r0 = __ldg(m.erow + slice0_ + sub_), r1 = __ldg(m.erow + slice0_ + sub_ + 1);
+    prefetch_l2(m.lidx + size_t(r0) * kSlice, (long long)(r1 - r0) * kSlice * 2);
+  }
   const Phys& ph = CASE_PH;
-  const int nu = it_.ncell + it_.nh;
-  int4* sL = smem + swz_chunks<1>(nu);
-  stage_records<1>(smem, s.QF, it_, m.hcell + it_.hoff, it_.nh);
-  stage_records<2>(sL, s.LF, it_, m.chcell + it_.choff, it_.nch);
+  const int pq = plane_len(max_u, 1), pl = plane_len(max_cu, 2);
+  int4* sL = sQ + pq;
+  stage_records<1, 1>(sQ, pq, s.QF, it_, m.hcell + it_.hoff, it_.nh);
+  stage_records<2, 2>(sL, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
-  const long long Q = m.Q;
   // limitAsgs's dt: this step's, or outside a step the control block's
   const double dt_sgs = (mode & 1) ? s.ctl->dt : s.ctl->dt_sgs;
   double cmax = 0.0;
   int anynan = 0;
-  STAGED_ROUNDS_BEGIN(G, PF_ENDF)
-  long long b = 0, e = 0, q0 = 0, q1 = 0;
-  LRecF Li;
+  SLICES_BEGIN(G)
+  int n = 0;
   float4 qi = make_float4(0.f, 0.f, 0.f, 0.f);
+  const unsigned short* eidx = m.lidx + (threadIdx.x & 31);
   if (valid) {
-    b = m.off[i];
-    e = m.off[i + 1];
-    q0 = m.qoff[i];
-    q1 = m.qoff[i + 1];
-    smem_LF(sL, loc_, Li);
-    qi = reinterpret_cast<const float4*>(smem)[loc_];
+    n = m.cnt[i].x;
+    eidx += size_t(__ldg(m.erow + slice_)) * 32;
+    qi = reinterpret_cast<const float4*>(sQ)[loc_];
   }
   float vv2 = 0.0f;
-  double cfl = 0.0;
-  for (long long k = b + lane; k < e; k += G) {
-    const float4 qj = reinterpret_cast<const float4*>(smem)[__ldg(m.lidx + k)];
-    const float dp = qj.y - qi.y;
-    const float v_avg = 0.5f * (qi.z + qj.z);
-    const float beta = 0.5f * (qi.w + qj.w);
-    const float gr = qj.x - qi.x - v_avg * dp * beta;
-    vv2 = fmaxf(vv2, fabsf(gr));
-  }
-  for (long long q = q0 + lane; q < q1; q += G) {
-    const int jl = __ldg(m.clidx + q);
-    const float* h = m.qg32 + q;
-    const float un[3] = {__ldg(h), __ldg(h + Q), __ldg(h + 2 * Q)};
-    const float area = __ldg(h + 3 * Q);
-    LRecF Lj;
-    smem_LF(sL, jl, Lj);
-    const float undA = 0.5f * area * ((Li.u[0] * un[0] + Li.u[1] * un[1] + Li.u[2] * un[2]) +
-                                      (Lj.u[0] * un[0] + Lj.u[1] * un[1] + Lj.u[2] * un[2]));
-    cfl += double(fabsf(undA)) + double(area) * (0.5 * (double(Li.sos) + double(Lj.sos)));
-  }
+  for (int r = part_; r < n; r += kIdxBatch * parts_) {
+    int jl[kIdxBatch];  // (past the last row: the cell itself, remainder zero)
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) vv2 = fmaxf(vv2, __shfl_xor_sync(0xffffffffu, vv2, o));
-  cfl = group_sum<G>(cfl);
-  if (valid && lane == 0) {
-    anynan |= cell_props_f(ph, m, s, i, Li, vv2, dt_sgs);
-    cfl += cfl_bf(m, i, double(Li.u[0]), double(Li.u[1]), double(Li.u[2]), double(Li.sos));
+    for (int b = 0; b < kIdxBatch; ++b) jl[b] = (r + b * parts_ < n) ? __ldg(eidx + (r + b * parts_) * 32) : loc_;
+#pragma unroll
+    for (int b = 0; b < kIdxBatch; ++b) {
+      const float4 qj = reinterpret_cast<const float4*>(sQ)[jl[b]];
+      const float dp = qj.y - qi.y;
+      const float v_avg = 0.5f * (qi.z + qj.z);
+      const float beta = 0.5f * (qi.w + qj.w);
+      const float gr = qj.x - qi.x - v_avg * dp * beta;
+      vv2 = fmaxf(vv2, fabsf(gr));
+    }
+  }
+  double v[2] = {double(vv2), 0.0};  // the remainder's maximum, the CFL sum
+  LRecF Li;
+  if (valid) smem_LF(sL, pl, loc_, Li);
+#pragma unroll 1
+  while (rows.left > 0) {
+    float2 h[2];
+    const int jl = rows.next(parts_, h);
+    LRecF Lj;
+    smem_LF(sL, pl, jl, Lj);
+    const float undA = 0.5f * h[1].y * ((Li.u[0] * h[0].x + Li.u[1] * h[0].y + Li.u[2] * h[1].x) +
+                                        (Lj.u[0] * h[0].x + Lj.u[1] * h[0].y + Lj.u[2] * h[1].x));
+    v[1] += double(fabsf(undA)) + double(h[1].y) * (0.5 * (double(Li.sos) + double(Lj.sos)));
+  }
+  combine_parts<2, true>(v, smem, kSumBytes<double>(2), part_, parts_, t_ + spr_ < nsl_);
+  if (valid && part_ == 0) {
+    smem_LF(sL, pl, loc_, Li);
+    anynan |= cell_props_f(ph, m, s, i, Li, float(v[0]), dt_sgs);
+    const double cfl = v[1] + cfl_bf(m, i, double(Li.u[0]), double(Li.u[1]), double(Li.u[2]), double(Li.sos));
     cmax = fmax(cmax, cfl * (0.5 * 1.0 * __ldg(m.inv_vol + i)));
   }
-  STAGED_ROUNDS_END
-  sh_cfl[threadIdx.x] = cmax;
-  sh_nan[threadIdx.x] = anynan;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (int(threadIdx.x) < w) {
-      sh_cfl[threadIdx.x] = fmax(sh_cfl[threadIdx.x], sh_cfl[threadIdx.x + w]);
-      sh_nan[threadIdx.x] |= sh_nan[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const int np = CASE_NITEMS;
-    s.red[it_.idx] = sh_cfl[0];
-    s.red[np + it_.idx] = double(sh_nan[0]);
-    __threadfence();
-    const unsigned int done = atomicAdd(&s.ctl->blocks_done, 1u);
-    am_last = (done == unsigned(np) - 1u);
-  }
-  __syncthreads();
-  if (am_last) {
-    __threadfence();
-    finalize_ctl(s.ctl, s.red, ph.dt_mode, ph.dt_max, mode, CASE_NITEMS);
-  }
+  if (t_ + spr_ < nsl_) ROWS_START(m.qrow, y, m.clidx, m.qg32, t_ + spr_)
+  SLICES_END
+  item_partial(cmax, anynan, s, ph, it_.idx, CASE_NITEMS, mode);
   STAGED_LOOP_END
-#undef PF_ENDF
 }
 
 #endif
