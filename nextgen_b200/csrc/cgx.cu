@@ -131,6 +131,18 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(unsigned(e - a)) : "memory");
 }
 
+// ---- overlapped launches ---------------------------------------------------
+// The step's kernels are launched with programmatic stream serialization: a
+// kernel's CTAs may start while the last CTAs of the one before still run.
+// Until after_previous() returns, i.e. until that kernel and with it all
+// earlier work is complete and visible, they touch only what no kernel of a
+// step writes: the mesh and the work list (their first rows are on their way
+// into L2 meanwhile).  Every CTA with work calls it.  launch_next() lets the
+// next kernel start.  One FP64 step of 8^3 cells 0.076 -> 0.064 ms, 48^3 0.604 ->
+// 0.595, a batch of 12 boxes 1.5 % faster; nothing at 128^3.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- row streams ---------------------------------------------------------
 // A warp walks the rows of one slice, one of `parts` warps taking rows part,
 // part + parts, ...  A lane's values of a row are stored in C chunks of type T
@@ -399,6 +411,7 @@ __host__ __device__ constexpr int kSumBytes(int NV) {
 // DIRECT (a template parameter of every step kernel): one case passed by value
 // in `dcase`, items read from its mesh's own item table.
 #define STAGED_LOOP_BEGIN(G)                                                   \
+  launch_next();                                                               \
   const int n_items_ = DIRECT ? dcase.nitems : *nitems;                        \
   for (int v_ = blockIdx.x; v_ < n_items_; v_ += gridDim.x) {                  \
     const Item it_ = DIRECT ? dcase.m.items[v_] : items[v_];                   \
@@ -487,6 +500,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   ROWS_START(m.erow, x, m.lidx, m.en, 0)
   double* const mf = DIRECT ? s.mf : nullptr;  // (a batch's cases carry no scalars)
   const int pl = plane_len(max_u, kEChunks);
+  after_previous();
   stage_records<kEChunks, 4>(sE, pl, s.L, it_, m.hcell + it_.hoff, it_.nh);
   const double K = CASE_PH.gamma * CASE_PH.invgm1;
   stage_wait();
@@ -537,6 +551,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 3 : G <= 8 ? 2 : 1) k_
   double* const mf = DIRECT ? s.mf : nullptr;
   const int pl = plane_len(max_cu, 4), pv = plane_len(max_cu, 8);
   int4* sV = sL + 4 * pl;
+  after_previous();
   stage_records<4, 4>(sL, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_records<8, 8>(sV, pv, s.V, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
@@ -678,6 +693,8 @@ template <bool DIRECT>
 __global__ void __launch_bounds__(kItemCells) k_rk_prim(CASE_ARGS, int nw, double w0, double w1, double w2,
                                                  double dt_arg, int writeQ) {
   // a single case takes its cells in order, a batch's case its items
+  launch_next();
+  after_previous();
   const int n_items_ = DIRECT ? 0 : *nitems;
   for (int v_ = blockIdx.x; DIRECT ? v_ == int(blockIdx.x) : v_ < n_items_; v_ += gridDim.x) {
     Item it_{};
@@ -737,6 +754,7 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad(CASE_ARGS) {
   Rows<768, double, 3> rows;
   ROWS_START(m.grow, z, m.cglidx, m.gc, 0)
   const int pl = plane_len(max_cu, 2);
+  after_previous();
   stage_records<2, 4>(smem, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
   const double2* su = reinterpret_cast<const double2*>(smem);
@@ -967,6 +985,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 5 : G <= 8 ? 3 : 1) k_
   const Phys& ph = CASE_PH;
   const int pq = plane_len(max_u, 2), pl = plane_len(max_cu, 4);
   int4* sL = sQ + 2 * pq;
+  after_previous();
   stage_records<2, 2>(sQ, pq, s.Q, it_, m.hcell + it_.hoff, it_.nh);
   stage_records<4, 4>(sL, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
@@ -2543,6 +2562,7 @@ struct Runner {
   cgx_precision prec = CGX_FP64;
   int max_union = 0;            // staging sizes: largest unions over the cases
   int max_cunion = 0;
+  bool overlap = true;          // overlapped launches (off while events time single kernels)
   std::atomic<long long>* launches = nullptr;
   SourceCfg* src = nullptr;     // source terms (single-case solvers only)
 };
@@ -2597,6 +2617,22 @@ int launch_check(const Runner& R, int nk) {
   return CGX_OK;
 }
 
+// Launch one of the step's kernels (see launch_next / after_previous).
+template <class... P, class... A>
+void launch_step(const Runner& R, void (*kernel)(P...), int grid, int block, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = R.stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = R.overlap ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 #define RARGS R.cases, R.items, R.nitems, R.dcase, R.max_union, R.max_cunion
 
 // the staged kernels take one item per CTA
@@ -2628,10 +2664,10 @@ inline size_t smem_comp(const Runner& R) {
 int enqueue_prim(const Runner& R, int nw, const double* w, double dt_arg, bool writeQ) {
   const double w0 = w ? w[0] : 0.0, w1 = w ? w[1] : 0.0, w2 = w ? w[2] : 0.0;
   if (R.direct)
-    k_rk_prim<true><<<(R.dcase.m.N + kItemCells - 1) / kItemCells, kItemCells, 0, R.stream>>>(
-        RARGS, nw, w0, w1, w2, dt_arg, writeQ ? 1 : 0);
+    launch_step(R, k_rk_prim<true>, (R.dcase.m.N + kItemCells - 1) / kItemCells, kItemCells, 0, RARGS, nw, w0, w1, w2,
+                dt_arg, writeQ ? 1 : 0);
   else
-    k_rk_prim<false><<<R.grid, kItemCells, 0, R.stream>>>(RARGS, nw, w0, w1, w2, dt_arg, writeQ ? 1 : 0);
+    launch_step(R, k_rk_prim<false>, R.grid, kItemCells, 0, RARGS, nw, w0, w1, w2, dt_arg, writeQ ? 1 : 0);
   return launch_check(R, 1);
 }
 
@@ -2640,30 +2676,30 @@ int enqueue_prim(const Runner& R, int nw, const double* w, double dt_arg, bool w
 template <int G, bool MIX, bool DIRECT>
 void launch_grad_d(const Runner& R) {
   if (MIX)
-    k_grad_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_grad<G>(R), R.stream>>>(RARGS);
+    launch_step(R, k_grad_f<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_grad<G>(R), RARGS);
   else
-    k_grad<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_grad<G>(R), R.stream>>>(RARGS);
+    launch_step(R, k_grad<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_grad<G>(R), RARGS);
 }
 template <int G, bool MIX, bool DIRECT>
 void launch_ext_d(const Runner& R, int st) {
   if (MIX)
-    k_rhs_ext_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_ext<G>(R), R.stream>>>(RARGS, st);
+    launch_step(R, k_rhs_ext_f<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_ext<G>(R), RARGS, st);
   else
-    k_rhs_ext<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_ext<G>(R), R.stream>>>(RARGS, st);
+    launch_step(R, k_rhs_ext<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_ext<G>(R), RARGS, st);
 }
 template <int G, bool MIX, bool DIRECT>
 void launch_comp_d(const Runner& R, int st) {
   if (MIX)
-    k_rhs_comp_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_comp<G>(R), R.stream>>>(RARGS, st);
+    launch_step(R, k_rhs_comp_f<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_comp<G>(R), RARGS, st);
   else
-    k_rhs_comp<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_comp<G>(R), R.stream>>>(RARGS, st);
+    launch_step(R, k_rhs_comp<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_comp<G>(R), RARGS, st);
 }
 template <int G, bool MIX, bool DIRECT>
 void launch_end_d(const Runner& R, int mode) {
   if (MIX)
-    k_step_end_f<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_end<G>(R), R.stream>>>(RARGS, mode);
+    launch_step(R, k_step_end_f<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_end<G>(R), RARGS, mode);
   else
-    k_step_end<G, DIRECT><<<grid_staged(R), kThreads<G>(), smem_end<G>(R), R.stream>>>(RARGS, mode);
+    launch_step(R, k_step_end<G, DIRECT>, grid_staged(R), kThreads<G>(), smem_end<G>(R), RARGS, mode);
 }
 
 // The staged kernels may use more than the default 48 KB of dynamic shared
@@ -3037,14 +3073,16 @@ bool fixed_tune(Tune* t) {
   return true;
 }
 
-int autotune(Runner& R, long long ncells) {
+int autotune(Runner& run, long long ncells) {
+  Runner R = run;
+  R.overlap = false;
   const int bucket = tune_bucket(ncells, R.prec);
-  if (fixed_tune(&R.tune)) return CGX_OK;
+  if (fixed_tune(&run.tune)) return CGX_OK;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(bucket);
     if (it != g_tune_cache.end()) {
-      R.tune = it->second;
+      run.tune = it->second;
       return CGX_OK;
     }
   }
@@ -3095,7 +3133,7 @@ int autotune(Runner& R, long long ncells) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
-  R.tune = best;
+  run.tune = best;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune_cache[bucket] = best;
   return CGX_OK;
@@ -5208,7 +5246,9 @@ static int ensure_pgraph(cgx_solver* s) {
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   const long long before = s->launches.load();
-  int rc = enqueue_step(s->run, s->pev);
+  Runner plain = s->run;
+  plain.overlap = false;
+  int rc = enqueue_step(plain, s->pev);
   cudaError_t ec = cudaStreamEndCapture(s->stream, &g);
   s->launches = before;
   if (rc || ec != cudaSuccess) cudaGetLastError();  // a failed capture leaves no error behind
@@ -5273,16 +5313,18 @@ extern "C" int cgx_kernel_times(cgx_solver* s, int reps, double ms[6]) {
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
+  Runner plain = s->run;
+  plain.overlap = false;
   int rc = CGX_OK;
   for (int which = 0; which < 6 && rc == CGX_OK; ++which) {
     CK(cudaEventRecord(e0, s->stream));
     for (int r = 0; r < reps && rc == CGX_OK; ++r) {
-      if (which == 0) rc = enqueue_rhs(s->run, 0);
-      else if (which == 1) rc = enqueue_prim(s->run, 3, kRkW[2], 0.0, true);
-      else if (which == 2) rc = enqueue_grad(s->run);
-      else if (which == 3) rc = enqueue_step_end(s->run, 0);
-      else if (which == 4) rc = ext_var(s->run, s->run.tune.g_ext, 0);
-      else rc = comp_var(s->run, s->run.tune.g_comp, 0);
+      if (which == 0) rc = enqueue_rhs(plain, 0);
+      else if (which == 1) rc = enqueue_prim(plain, 3, kRkW[2], 0.0, true);
+      else if (which == 2) rc = enqueue_grad(plain);
+      else if (which == 3) rc = enqueue_step_end(plain, 0);
+      else if (which == 4) rc = ext_var(plain, plain.tune.g_ext, 0);
+      else rc = comp_var(plain, plain.tune.g_comp, 0);
     }
     CK(cudaEventRecord(e1, s->stream));
     CK(cudaEventSynchronize(e1));

@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 8 : G <= 8 ? 4 : 1) k_
   ROWS_START(m.erow, x, m.lidx, m.en32, 0)
   double* const mf = DIRECT ? s.mf : nullptr;
   const int pl = plane_len(max_u, 2);
+  after_previous();
   stage_records<2, 2>(sL, pl, s.LF, it_, m.hcell + it_.hoff, it_.nh);
   const double h_ref = CASE_PH.h_ref;
   stage_wait();
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   double* const mf = DIRECT ? s.mf : nullptr;
   const int pl = plane_len(max_cu, 2), pv = plane_len(max_cu, 4);
   int4* sV = sL + 2 * pl;
+  after_previous();
   stage_records<2, 2>(sL, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_records<4, 4>(sV, pv, s.VF, it_, m.chcell + it_.choff, it_.nch);
   const double h_ref = CASE_PH.h_ref;
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad_f(CASE_ARGS) {
   Rows<384, float, 3> rows;
   ROWS_START(m.grow, z, m.cglidx, m.gc32, 0)
   const int pl = plane_len(max_cu, 1);
+  after_previous();
   stage_records<1, 2>(smem, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
   const float4* su = reinterpret_cast<const float4*>(smem);
@@ -387,6 +390,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   const Phys& ph = CASE_PH;
   const int pq = plane_len(max_u, 1), pl = plane_len(max_cu, 2);
   int4* sL = sQ + pq;
+  after_previous();
   stage_records<1, 1>(sQ, pq, s.QF, it_, m.hcell + it_.hoff, it_.nh);
   stage_records<2, 2>(sL, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
