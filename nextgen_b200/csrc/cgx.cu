@@ -2602,7 +2602,7 @@ struct cgx_solver {
   cudaStream_t ostream = nullptr;
   cudaEvent_t oev = nullptr;
   cudaEvent_t pev[9] = {};
-  std::unique_ptr<cgx_staging::Staging> staging;  // for pageable caller arrays, made on first use
+  std::unique_ptr<cgx_staging::Staging> staging;  // for pageable caller arrays, during a call
   std::atomic<long long> launches{0};
   SourceCfg src;
   std::vector<BcZone> bc;   // boundary conditions per zone (host copy of sd.bc)
@@ -4237,8 +4237,8 @@ extern "C" int cgx_solver_destroy(cgx_solver* s) {
 
 // Copies between the caller's host arrays and the device.  Page-locked
 // (cudaMallocHost or registered) arrays go straight to the copy engine;
-// pageable ones, such as a host solver's new[] arrays, go through the
-// solver's two pinned staging chunks with the host-side copy on all threads,
+// pageable ones, such as a host solver's new[] arrays, go through two
+// pinned staging chunks with the host-side copy on all threads,
 // which is several times faster than a pageable cudaMemcpy.
 static bool page_locked(const void* p) {
   cudaPointerAttributes a;
@@ -4261,6 +4261,13 @@ static int staging_of(cgx_solver* s, cgx_staging::Staging** st) {
   *st = s->staging.get();
   return CGX_OK;
 }
+
+// Gives the pinned chunks that a call took for its copies back at its end
+// (for other solvers, and for mesh set-up), once they are idle.
+struct StagingLease {
+  cgx_solver* s;
+  ~StagingLease() { s->staging.reset(); }
+};
 
 static int host_to_device(cgx_solver* s, void* dst, const void* src, size_t bytes) {
   if (bytes < (size_t(4) << 20) || page_locked(src)) {
@@ -4298,6 +4305,7 @@ static int upload_stage(cgx_solver* s, const double* a, const double* u, const d
 extern "C" int cgx_set_state(cgx_solver* s, const double* rho, const double* u, const double* rhoE) {
   if (!s || !rho || !u || !rhoE) return fail(CGX_E_ARG, "cgx_set_state: null argument");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   int rc = upload_stage(s, rho, u, rhoE);
   if (rc) return rc;
   const int N = s->mesh->N;
@@ -4311,6 +4319,7 @@ extern "C" int cgx_set_state(cgx_solver* s, const double* rho, const double* u, 
 extern "C" int cgx_set_state_primitive(cgx_solver* s, const double* rho, const double* u, const double* p) {
   if (!s || !rho || !u || !p) return fail(CGX_E_ARG, "cgx_set_state_primitive: null argument");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   int rc = upload_stage(s, rho, u, p);
   if (rc) return rc;
   const int N = s->mesh->N;
@@ -4324,6 +4333,7 @@ extern "C" int cgx_set_state_primitive(cgx_solver* s, const double* rho, const d
 extern "C" int cgx_get_state(cgx_solver* s, double* rho, double* u, double* rhoE) {
   if (!s) return fail(CGX_E_ARG, "cgx_get_state: null argument");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   const int N = s->mesh->N;
   k_state_out<<<(N + 255) / 256, 256, 0, s->stream>>>(N, s->mesh->d_perm, s->d_stage, s->sd);
   int rc = launch_check(s->run, 1);
@@ -4365,6 +4375,7 @@ extern "C" int cgx_set_scalars(cgx_solver* s, int nsc, const double* sc) {
       if (bc_no_scalars(z.kind))
         return fail(CGX_E_STATE, "cgx_set_scalars: CBC and HOOK boundary zones carry no transport scalars");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   CK(cudaStreamSynchronize(s->stream));
   const size_t N = size_t(s->mesh->N);
   StateDev& sd = s->sd;
@@ -4418,6 +4429,7 @@ extern "C" int cgx_get_scalars(cgx_solver* s, double* sc) {
   const int nsc = s->sd.nsc;
   if (nsc == 0) return fail(CGX_E_STATE, "cgx_get_scalars: the solver has no transport scalars");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   const int N = s->mesh->N;
   k_scalars_io<<<(N + 255) / 256, 256, 0, s->stream>>>(N, nsc, s->mesh->d_perm, s->d_stage, s->sd, 1, 0);
   int rc = launch_check(s->run, 1);
@@ -4433,6 +4445,7 @@ extern "C" int cgx_get_rhs_sc(cgx_solver* s, int rk_stage, double* rhs_sc) {
   const int nsc = s->sd.nsc;
   if (nsc == 0) return fail(CGX_E_STATE, "cgx_get_rhs_sc: the solver has no transport scalars");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   const int N = s->mesh->N;
   k_scalars_io<<<(N + 255) / 256, 256, 0, s->stream>>>(N, nsc, s->mesh->d_perm, s->d_stage, s->sd, 2,
                                                        rk_stage - 1);
@@ -4470,6 +4483,7 @@ extern "C" int cgx_set_frame_rotation(cgx_solver* s, const double rev[3], const 
   const bool on = rev[0] != 0.0 || rev[1] != 0.0 || rev[2] != 0.0;
   if (on && !x_cv) return fail(CGX_E_ARG, "cgx_set_frame_rotation: the cell centroids are needed");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   CK(cudaStreamSynchronize(s->stream));
   const size_t N = size_t(s->mesh->N);
   if (on) {
@@ -4505,6 +4519,7 @@ extern "C" int cgx_set_frame_rotation(cgx_solver* s, const double rev[3], const 
 extern "C" int cgx_set_source(cgx_solver* s, const cgx_source* src) {
   if (!s) return fail(CGX_E_ARG, "cgx_set_source: null solver");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   CK(cudaStreamSynchronize(s->stream));
   SourceCfg& c = s->src;
   const cgx_source none{};
@@ -5009,6 +5024,7 @@ extern "C" int cgx_calc_rhs(cgx_solver* s, double* rhs_out, double time, int rk_
   if (rk_stage < 1 || rk_stage > 3) return fail(CGX_E_ARG, "rk_stage must be 1..3");
   if (!s->inited) return fail(CGX_E_STATE, "cgx_init_complete not called");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   int rc = enqueue_rhs(s->run, rk_stage - 1, &time);
   if (rc) return rc;
   if (rhs_out) {
@@ -5162,6 +5178,7 @@ extern "C" int cgx_step_out(cgx_solver* s, int nsteps, double* rho, double* u, d
   if (!s->inited) return fail(CGX_E_STATE, "cgx_init_complete not called");
   if (nsteps < 1) return fail(CGX_E_ARG, "nsteps < 1");
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   int rc;
   if (nsteps > 1 && (rc = cgx_step(s, nsteps - 1))) {
     if (rc == CGX_E_NAN) cgx_get_state(s, rho, u, rhoE);
@@ -5364,6 +5381,7 @@ extern "C" int cgx_totals(cgx_solver* s, double out[5]) {
 
 static int diag(cgx_solver* s, int what, int k, double* out) {
   CK(cudaSetDevice(s->mesh->device));
+  const StagingLease lease{s};
   const int N = s->mesh->N;
   k_diag_out<<<(N + 255) / 256, 256, 0, s->stream>>>(N, s->mesh->d_perm, s->d_stage, s->sd, what, 0, s->ph.R, s->ph.p_ref);
   int rc = launch_check(s->run, 1);

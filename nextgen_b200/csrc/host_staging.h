@@ -11,6 +11,8 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 namespace cgx_staging {
 
@@ -24,31 +26,91 @@ inline void par_memcpy(void* dst, const void* src, size_t bytes) {
   }
 }
 
+constexpr size_t kChunk = size_t(64) << 20;
+
+// The two pinned chunks of a Staging and the events of their last copies.
+// Page-locking 128 MiB takes 60 to 100 ms, most of the set-up of a small mesh
+// and of a solver's first pageable copy, so chunks that were given back are
+// kept for the next user: at most kKept pairs per process, freed beyond that.
+// A pair belongs to one Staging at a time and comes back idle (its stream
+// synchronised); the list is guarded for use from several threads.
+struct Chunks {
+  int device = -1;
+  char* pin[2] = {nullptr, nullptr};
+  cudaEvent_t done[2] = {nullptr, nullptr};
+
+  void free_all() {
+    for (int i = 0; i < 2; ++i) {
+      if (pin[i]) cudaFreeHost(pin[i]);
+      if (done[i]) cudaEventDestroy(done[i]);
+    }
+  }
+};
+
+constexpr size_t kKept = 2;
+struct ChunkPool {
+  std::mutex mu;
+  std::vector<Chunks> idle;
+};
+inline ChunkPool& chunk_pool() {
+  static ChunkPool* p = new ChunkPool();  // outlives every static user
+  return *p;
+}
+
+// a pair for the current device: a kept one that is still valid (a reset of
+// the device takes it away), or a new one
+inline cudaError_t take_chunks(Chunks* c) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  {
+    ChunkPool& p = chunk_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    for (size_t i = p.idle.size(); i-- > 0;) {
+      if (p.idle[i].device != device) continue;
+      Chunks k = p.idle[i];
+      p.idle.erase(p.idle.begin() + long(i));
+      cudaPointerAttributes a0{}, a1{};
+      if (cudaPointerGetAttributes(&a0, k.pin[0]) == cudaSuccess && a0.type == cudaMemoryTypeHost &&
+          cudaPointerGetAttributes(&a1, k.pin[1]) == cudaSuccess && a1.type == cudaMemoryTypeHost) {
+        *c = k;
+        return cudaSuccess;
+      }
+      cudaGetLastError();  // gone with its context
+    }
+  }
+  c->device = device;
+  for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+    e = cudaMallocHost(reinterpret_cast<void**>(&c->pin[i]), kChunk);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done[i], cudaEventDisableTiming);
+  }
+  return e;
+}
+
+inline void give_back(const Chunks& c) {
+  ChunkPool& p = chunk_pool();
+  std::lock_guard<std::mutex> lk(p.mu);
+  if (c.pin[0] && c.pin[1] && c.done[0] && c.done[1] && p.idle.size() < kKept) {
+    p.idle.push_back(c);
+  } else {
+    Chunks k = c;
+    k.free_all();
+  }
+}
+
 class Staging {
  public:
-  static constexpr size_t kChunk = size_t(64) << 20;
-
   explicit Staging(cudaStream_t s) : s_(s) {}
   Staging(const Staging&) = delete;
   Staging& operator=(const Staging&) = delete;
 
   // pinned buffers and events; must succeed before put/get
-  cudaError_t init() {
-    for (int i = 0; i < 2; ++i) {
-      cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&pin_[i]), kChunk);
-      if (e != cudaSuccess) return e;
-      e = cudaEventCreateWithFlags(&done_[i], cudaEventDisableTiming);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-  }
+  cudaError_t init() { return take_chunks(&c_); }
 
   ~Staging() {
-    cudaStreamSynchronize(s_);  // no DMA may still target the buffers
-    for (int i = 0; i < 2; ++i) {
-      if (pin_[i]) cudaFreeHost(pin_[i]);
-      if (done_[i]) cudaEventDestroy(done_[i]);
-    }
+    // no DMA may still target the buffers; if that cannot be known, they stay
+    // with the process
+    if (cudaStreamSynchronize(s_) == cudaSuccess) give_back(c_);
   }
 
   // host -> device, asynchronous on the stream (src may be reused on return)
@@ -56,12 +118,12 @@ class Staging {
     const size_t nch = (bytes + kChunk - 1) / kChunk;
     for (size_t c = 0; c < nch; ++c) {
       const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-      cudaError_t e = cudaEventSynchronize(done_[c & 1]);  // the buffer's previous DMA
+      cudaError_t e = cudaEventSynchronize(c_.done[c & 1]);  // the buffer's previous DMA
       if (e != cudaSuccess) return e;
-      par_memcpy(pin_[c & 1], static_cast<const char*>(src) + off, len);
-      e = cudaMemcpyAsync(static_cast<char*>(dst) + off, pin_[c & 1], len, cudaMemcpyHostToDevice, s_);
+      par_memcpy(c_.pin[c & 1], static_cast<const char*>(src) + off, len);
+      e = cudaMemcpyAsync(static_cast<char*>(dst) + off, c_.pin[c & 1], len, cudaMemcpyHostToDevice, s_);
       if (e != cudaSuccess) return e;
-      e = cudaEventRecord(done_[c & 1], s_);
+      e = cudaEventRecord(c_.done[c & 1], s_);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -71,31 +133,36 @@ class Staging {
   // stream when given (the copies then follow st's earlier work)
   cudaError_t get(void* dst, const void* src, size_t bytes, cudaStream_t st = nullptr) {
     cudaStream_t q = st ? st : s_;
+    const cudaError_t e = get_on(q, dst, src, bytes);
+    if (e != cudaSuccess) cudaStreamSynchronize(q);  // leave no copy in flight behind an error
+    return e;
+  }
+
+ private:
+  cudaError_t get_on(cudaStream_t q, void* dst, const void* src, size_t bytes) {
     const size_t nch = (bytes + kChunk - 1) / kChunk;
     for (size_t c = 0; c < nch; ++c) {
       const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-      cudaError_t e = cudaMemcpyAsync(pin_[c & 1], static_cast<const char*>(src) + off, len,
+      cudaError_t e = cudaMemcpyAsync(c_.pin[c & 1], static_cast<const char*>(src) + off, len,
                                       cudaMemcpyDeviceToHost, q);
       if (e != cudaSuccess) return e;
-      e = cudaEventRecord(done_[c & 1], q);
+      e = cudaEventRecord(c_.done[c & 1], q);
       if (e != cudaSuccess) return e;
       if (c > 0 && (e = drain(static_cast<char*>(dst), c - 1, bytes)) != cudaSuccess) return e;
     }
     return nch > 0 ? drain(static_cast<char*>(dst), nch - 1, bytes) : cudaSuccess;
   }
 
- private:
   cudaError_t drain(char* dst, size_t c, size_t bytes) {
     const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-    const cudaError_t e = cudaEventSynchronize(done_[c & 1]);
+    const cudaError_t e = cudaEventSynchronize(c_.done[c & 1]);
     if (e != cudaSuccess) return e;
-    par_memcpy(dst + off, pin_[c & 1], len);
+    par_memcpy(dst + off, c_.pin[c & 1], len);
     return cudaSuccess;
   }
 
   cudaStream_t s_;
-  char* pin_[2] = {nullptr, nullptr};
-  cudaEvent_t done_[2] = {nullptr, nullptr};
+  Chunks c_;
 };
 
 }  // namespace cgx_staging
