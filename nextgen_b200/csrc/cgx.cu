@@ -2479,16 +2479,6 @@ int dupload(T** p, const std::vector<T, A>& v, size_t* acc, cgx_staging::Staging
   return dupload(p, v.data(), v.size(), st, acc);
 }
 
-inline uint64_t spread3(uint64_t x) {  // 21 bits -> every third bit
-  x &= 0x1fffff;
-  x = (x | x << 32) & 0x1f00000000ffffULL;
-  x = (x | x << 16) & 0x1f0000ff0000ffULL;
-  x = (x | x << 8) & 0x100f00f00f00f00fULL;
-  x = (x | x << 4) & 0x10c30c30c30c30c3ULL;
-  x = (x | x << 2) & 0x1249249249249249ULL;
-  return x;
-}
-
 }  // namespace
 
 struct cgx_mesh {
@@ -3316,6 +3306,39 @@ static int item_cells(int N) {
   return kSlice;
 }
 
+// Order p[0, n) so that every run of `block` cells is compact: the cells are
+// halved (at a multiple of `block`) across the longest side of their bounding
+// box until a run is left, whose cells then stand in index order.  With
+// block = 128 an item of a box of 100^3 cells reaches 759 cells on average and
+// 838 at most; runs of a Morton order of the same box, whose power-of-two boxes
+// do not hold 128 cells there, reached 874 and 1115 (on 64^3, where they do,
+// 697 and 779, here 697 and 729).
+static void bisect_cells(int* p, int n, const double* x, int block) {
+  while (n > block) {
+    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    for (int i = 0; i < n; ++i)
+      for (int k = 0; k < 3; ++k) {
+        const double v = x[3 * size_t(p[i]) + k];
+        lo[k] = std::min(lo[k], v);
+        hi[k] = std::max(hi[k], v);
+      }
+    int k = 0;
+    for (int c = 1; c < 3; ++c)
+      if (hi[c] - lo[c] > hi[k] - lo[k]) k = c;
+    const int left = ((n + block - 1) / block / 2) * block;
+    std::nth_element(p, p + left, p + n, [&](int a, int b) {
+      const double xa = x[3 * size_t(a) + k], xb = x[3 * size_t(b) + k];
+      return xa < xb || (xa == xb && a < b);
+    });
+    int* q = p;
+#pragma omp task firstprivate(q, left) if (n > 16384)
+    bisect_cells(q, left, x, block);
+    p += left;
+    n -= left;
+  }
+  std::sort(p, p + n);
+}
+
 // The order of a slice's entries: rows x 32 lanes, each lane's entries (the
 // range off[l], off[l+1] of idx) in any order, one per row from row 0 on.  The
 // 16-byte shared-memory reads of eight neighbouring lanes are served together
@@ -3403,32 +3426,18 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     for (int g = 0; g < ncv_g2 - N; ++g)
       if (d->icv_owner_g[g] < 0 || d->icv_owner_g[g] >= N) return bail(fail(CGX_E_ARG, "ghost owner out of range"));
     auto owner = [&](int idx) { return idx < N ? idx : d->icv_owner_g[idx - N]; };
-    // ---- renumbering (Morton order of x_cv)
+    // ---- renumbering: each work item's cells are a compact block of x_cv
+    const int icells = item_cells(N);
     std::vector<int>& perm = M->perm;
     perm.resize(N);
     std::iota(perm.begin(), perm.end(), 0);
     if (d->x_cv) {
-      double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-      for (int i = 0; i < N; ++i)
-        for (int k = 0; k < 3; ++k) {
-          lo[k] = std::min(lo[k], d->x_cv[3 * size_t(i) + k]);
-          hi[k] = std::max(hi[k], d->x_cv[3 * size_t(i) + k]);
-        }
-      std::vector<uint64_t> key(N);
-#pragma omp parallel for schedule(static)
-      for (int i = 0; i < N; ++i) {
-        uint64_t q[3];
-        for (int k = 0; k < 3; ++k) {
-          const double t = (hi[k] > lo[k]) ? (d->x_cv[3 * size_t(i) + k] - lo[k]) / (hi[k] - lo[k]) : 0.0;
-          q[k] = uint64_t(std::min(std::max(t, 0.0), 1.0) * 2097151.0);
-        }
-        key[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
-      }
-      std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return key[a] < key[b]; });
+#pragma omp parallel
+#pragma omp single
+      bisect_cells(perm.data(), N, d->x_cv, icells);
     }
     // ---- inside each work item cells are ordered by their extended faces,
     // most first (stable), so that the rows of a slice have few empty lanes
-    const int icells = item_cells(N);
     {
       int bad_ef = 0;
 #pragma omp parallel for schedule(static) reduction(| : bad_ef)
