@@ -265,18 +265,19 @@ __device__ __forceinline__ double4 smem_Q(const int4* sm, int pl, int j) {
 }
 
 // Skew-symmetric flux plus its symmetric "c" part (IdealGasSolverFlux.hpp:
-// 9-39 and 41-90) of the face a -> b, subtracted from the five sums and
-// returned as its mass flux.  The reference's two functions produce the same
-// terms; here they are grouped around the total mass flux M = mdot + dmdot:
+// 9-39 and 41-90) of the face a -> b.  The reference's two functions produce
+// the same terms; here they are grouped around the total mass flux
+// M = mdot + dmdot:
 //   F.rho = M
-//   F.ru  = p_f n + dp c + M uf + mdot_c du
+//   F.ru  = p_f n + dp c/2 + M uf + mdot_c du
 //   F.rE  = M h_f + mdot_c (dh + uf.du)
-// (mdot = rho_f uf.n, dmdot = uf.c drho + rho_f du.c, mdot_c = rho_f uf.c), on
-// the sums s = u_a + u_b = 2 uf and r = rho_f / 2, whose halves are exact.
-// Every term changes sign exactly under (a <-> b, n -> -n, c kept), so the
-// two cells of a face see exactly opposite fluxes.
-__device__ __forceinline__ double ext_flux_sub(double acc[5], const double n[3], const double c[3], const ERec& a,
-                                               double ha, const ERec& b, double K) {
+// (mdot = rho_f uf.n, dmdot = (uf.c drho + rho_f du.c)/2, mdot_c = rho_f uf.c/2).
+// F holds M and twice the others, on the sums s = u_a + u_b = 2 uf and r =
+// 1/(v_a + v_b) = rho_f/2, so that no halves are left (powers of two: the same
+// roundings); qr = rho_a/4.  Every term changes sign exactly under (a <-> b,
+// n -> -n, c kept), so the two cells of a face see exactly opposite fluxes.
+__device__ __forceinline__ void ext_flux(double F[5], const double n[3], const double c[3], const ERec& a, double qr,
+                                         double ha, const ERec& b, double K) {
   const double r = rcp_nr(a.v + b.v);
   double s[3], du[3];
 #pragma unroll
@@ -284,38 +285,29 @@ __device__ __forceinline__ double ext_flux_sub(double acc[5], const double n[3],
     s[d] = a.u[d] + b.u[d];
     du[d] = b.u[d] - a.u[d];
   }
-  const double sn = s[0] * n[0] + s[1] * n[1] + s[2] * n[2];
-  const double sc = s[0] * c[0] + s[1] * c[1] + s[2] * c[2];
-  const double duc = du[0] * c[0] + du[1] * c[1] + du[2] * c[2];
-  const double uaub = a.u[0] * b.u[0] + a.u[1] * b.u[1] + a.u[2] * b.u[2];
-  const double sdu = s[0] * du[0] + s[1] * du[1] + s[2] * du[2];
-  const double mdot_c = sc * r;
-  const double M = sn * r + (0.5 * (sc * (b.rho - a.rho)) + 2.0 * (r * duc));
+  const double duc = fma(du[2], c[2], fma(du[1], c[1], du[0] * c[0]));
+  const double w = fma(s[2], n[2], fma(s[1], n[1], fma(s[0], n[0], duc)));  // 2 (uf.n + du.c/2)
+  const double sc = fma(s[2], c[2], fma(s[1], c[1], s[0] * c[0]));
+  const double uaub = fma(a.u[2], b.u[2], fma(a.u[1], b.u[1], a.u[0] * b.u[0]));
+  const double sdu = fma(s[2], du[2], fma(s[1], du[1], s[0] * du[0]));
+  const double M = fma(r, w, sc * fma(0.25, b.rho, -qr));
+  const double mc = sc * r;  // 2 mdot_c
   const double hb = K * (b.p * b.v);
-  const double hp = 0.5 * (a.p + b.p), dp = b.p - a.p, hM = 0.5 * M;
-  const double dH = (hb - ha) + 0.5 * sdu;
-  acc[0] -= M;
+  const double ps = a.p + b.p, dp = b.p - a.p;
+  F[0] = M;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    acc[1 + d] -= hp * n[d];
-    acc[1 + d] -= dp * c[d];
-    acc[1 + d] -= hM * s[d];
-    acc[1 + d] -= mdot_c * du[d];
-  }
-  acc[4] -= hM * ((ha + hb) + uaub);
-  acc[4] -= mdot_c * dH;
-  return M;
+  for (int d = 0; d < 3; ++d) F[1 + d] = fma(M, s[d], fma(mc, du[d], fma(ps, n[d], dp * c[d])));
+  F[4] = fma(M, (ha + hb) + uaub, mc * fma(0.5, sdu, hb - ha));
 }
 
-// Compact closures (IdealGasSolverFlux.hpp:93-215) of the face a -> b, taken
-// from the five sums' negatives, i.e. acc += their value; returns the mass
-// flux they take from the face's.  The closures use the two cells' properties
+// Compact closures (IdealGasSolverFlux.hpp:93-215) of the face a -> b: F is what
+// they take from the face's flux.  The closures use the two cells' properties
 // and gradients only through their sums: vs holds V_a + V_b field by field.
 // With uf = (u_a + u_b)/2 and du = u_b - u_a the reference's differences of
 // squares are products: (|u_b|^2 - |u_a|^2)/2 = uf.du and (un_b^2 - un_a^2)/2 =
 // un_m dun.
-__device__ __forceinline__ double compact_flux_add(double acc[5], const double un_[3], double area, double aod,
-                                                   double delta, const LRec& a, const LRec& b, const VRec& vs) {
+__device__ __forceinline__ void compact_flux(double F[5], const double un_[3], double area, double aod, double delta,
+                                             const LRec& a, const LRec& b, const VRec& vs) {
   const double half_aod = 0.5 * aod;
   const double mu_area = 0.5 * vs.mu_total * area;
   const double mu_aod = vs.mu_total * half_aod;
@@ -353,14 +345,9 @@ __device__ __forceinline__ double compact_flux_add(double acc[5], const double u
   const double m = lf_drho + ap_dp;
   // along the normal: mu_aod dun/3 + lf_rho dun - mu_area trace
   const double kn = (mu_aod * (1.0 / 3.0) + lf_rho) * dun - mu_area * trace;
-  acc[0] += m;
+  F[0] = m;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    acc[1 + d] += mu_aod * du[d];
-    acc[1 + d] += m * uf[d];
-    acc[1 + d] += kn * un_[d];
-    acc[1 + d] += mu_area * gn[d];
-  }
+  for (int d = 0; d < 3; ++d) F[1 + d] = fma(mu_aod, du[d], fma(mu_area, gn[d], fma(kn, un_[d], m * uf[d])));
   const double hs = fmax(vs.symh * rho_m * aun * half_aod - k_aod, 0.0);
   const double pva = a.p * a.sp_vol, pvb = b.p * b.sp_vol;
   const double de = dh - (pvb - pva);
@@ -371,8 +358,7 @@ __device__ __forceinline__ double compact_flux_add(double acc[5], const double u
   e -= lf_drho * (0.5 * (pva + pvb));
   e += lf_rho * (de + un_m * dun);
   e += mu_area * (ufgn - un_m * trace);
-  acc[4] += e;
-  return -m;
+  F[4] = e;
 }
 
 // ===========================================================================
@@ -448,7 +434,7 @@ __host__ __device__ constexpr int kSumBytes(int NV) {
   }
 
 // Sum (MAXFIRST: the first value's maximum) of each lane's NV values over the
-// warps of its slice, in part order, left in part 0, through `bytes` (>= 32 NV
+// warps of its slice, in pairs of parts, left in part 0, through `bytes` (>= 32 NV
 // values) of shared memory per warp at `area`, which nothing else may be using.
 // All threads of the CTA call it; `again` (uniform) says that another round
 // follows.
@@ -465,16 +451,57 @@ __device__ __forceinline__ void combine_parts(T (&v)[NV], void* area, int bytes,
     }
     __syncthreads();
     if (part == 0) {
-#pragma unroll 1
-      for (int p = 1; p < parts; ++p) {
+      const auto add = [&](int p, int n) {
         const T* w = reinterpret_cast<const T*>(mine + p * bytes) + lane;
+        const T* x = reinterpret_cast<const T*>(mine + (p + 1) * bytes) + lane;
 #pragma unroll
-        for (int c = 0; c < NV; ++c) v[c] = (MAXFIRST && c == 0) ? fmax(v[c], w[0]) : v[c] + w[c * 32];
-      }
+        for (int c = 0; c < NV; ++c) {
+          if (MAXFIRST && c == 0)
+            v[c] = fmax(v[c], n == 2 ? fmax(w[0], x[0]) : w[0]);
+          else
+            v[c] += n == 2 ? w[c * 32] + x[c * 32] : w[c * 32];
+        }
+      };
+      add(1, 1);
+#pragma unroll 1
+      for (int p = 2; p + 1 < parts; p += 2) add(p, 2);
+      if (parts > 2 && (parts & 1)) add(parts - 1, 1);
     }
     if (again) __syncthreads();
   }
 }
+
+// A lane's sums over its rows are taken in blocks of a few rows (the first one
+// shorter): a block's sum is added to the earlier blocks', which wait in the
+// lane's slot of the warp's area for combine_parts (NV values, 32 apart).  In
+// one chain of up to 80 rows every entry would be rounded at the size of the
+// whole running sum.  Against 80-bit sums over sum |F| (a 46^3 box, one warp per
+// slice): momentum 1.1e-16 with each of a flux's terms added to one chain by
+// itself, 5.7e-17 so, where 16 lanes and a butterfly gave 6.0e-17; gradient
+// 1.2e-16 in one chain, 8.7e-17 so.  128^3: ext 1.47 ms (1.44 term by term),
+// gradient 0.269 (0.267).
+constexpr int kExtBlock = 8, kGradBlock = 5;
+template <int NV, class T>
+struct BlockSums {
+  T* kept;
+  bool any = false;
+  __device__ __forceinline__ BlockSums(void* area, int bytes)
+      : kept(reinterpret_cast<T*>(static_cast<char*>(area) + (int(threadIdx.x) >> 5) * bytes) + (threadIdx.x & 31)) {}
+  __device__ __forceinline__ void put(T (&v)[NV]) {
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      kept[c * 32] = any ? kept[c * 32] + v[c] : v[c];
+      v[c] = T(0);
+    }
+    any = true;
+  }
+  __device__ __forceinline__ void add_to(T (&v)[NV]) const {
+    if (any) {
+#pragma unroll
+      for (int c = 0; c < NV; ++c) v[c] += kept[c * 32];
+    }
+  }
+};
 
 // calcRhsBase, cell-centric, in two passes over each cell's face list:
 //   k_rhs_ext : rhs[i] = -sum over all of i's extended faces of the skew +
@@ -485,7 +512,7 @@ __device__ __forceinline__ void combine_parts(T (&v)[NV], void* area, int bytes,
 // reversed (n -> -n, unit_n -> -unit_n, c kept), which gives the negated flux.
 //
 // k_rhs_ext streams 50 B per directed entry (about 80 a cell) and is bound by
-// HBM: 128^3 jittered cells 1.44 ms, 6.0 TB/s of rows (with an entry's six values
+// HBM: 128^3 jittered cells 1.47 ms, 5.9 TB/s of rows (with an entry's six values
 // in planes of their own and G neighbouring lanes per cell, whose sums 40
 // shuffles a cell combined, 1.73 ms; 200^3 7.95 ms, where each CTA's seven
 // streams also missed the TLB).  A ring of rows in shared memory, filled by
@@ -502,18 +529,18 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   const int pl = plane_len(max_u, kEChunks);
   after_previous();
   stage_records<kEChunks, 4>(sE, pl, s.L, it_, m.hcell + it_.hoff, it_.nh);
-  const double K = CASE_PH.gamma * CASE_PH.invgm1;
+  const double K = CASE_PH.gogm1;
   stage_wait();
   SLICES_BEGIN(G)
   ERec Ei;
-  double hi = 0.0;
+  double hi = 0.0, qr = 0.0;
   if (valid) {
     smem_E(sE, pl, loc_, Ei);
     hi = K * (Ei.p * Ei.v);
+    qr = 0.25 * Ei.rho;
   }
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  size_t k = 0;  // the entry's place in mf
-  if (mf && valid) k = (size_t(__ldg(m.erow + slice_)) + part_) * 32 + (threadIdx.x & 31);
+  BlockSums<5, double> blocks(smem, kSumBytes<double>(5));
 #pragma unroll 1
   while (rows.left > 0) {
     double2 g[3];
@@ -521,17 +548,19 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
     ERec Ej;
     smem_E(sE, pl, jl, Ej);
     const double n[3] = {g[0].x, g[0].y, g[1].x}, c[3] = {g[1].y, g[2].x, g[2].y};
-    const double M = ext_flux_sub(acc, n, c, Ei, hi, Ej, K);
-    if (mf) {  // mf[ief] of calcRhsBase, for calcRhsScalars
-      mf[k] = M;
-      k += 32 * parts_;
-    }
+    double F[5];
+    ext_flux(F, n, c, Ei, qr, hi, Ej, K);
+    if (mf) mf[rows.idx - m.lidx - kSlice * parts_] = F[0];  // mf[ief] of calcRhsBase, for calcRhsScalars
+#pragma unroll
+    for (int q = 0; q < 5; ++q) acc[q] -= F[q];
+    if (rows.left % kExtBlock == 0 && rows.left > 0) blocks.put(acc);
   }
+  blocks.add_to(acc);
   combine_parts(acc, smem, kSumBytes<double>(5), part_, parts_, t_ + spr_ < nsl_);
   if (valid && part_ == 0) {
     double* r = s.rhs + size_t(stage) * 5 * m.N;
 #pragma unroll
-    for (int c = 0; c < 5; ++c) r[size_t(c) * m.N + i] = acc[c];
+    for (int c = 0; c < 5; ++c) r[size_t(c) * m.N + i] = c == 0 ? acc[0] : 0.5 * acc[c];
   }
   if (t_ + spr_ < nsl_) ROWS_START(m.erow, x, m.lidx, m.en, t_ + spr_)
   SLICES_END
@@ -570,11 +599,14 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 3 : G <= 8 ? 2 : 1) k_
     VRec Vs;
     smem_V_sum(sV, pv, loc_, jl, Vs);
     const double un[3] = {h[0].x, h[0].y, h[1].x};
-    const double dm = compact_flux_add(acc, un, h[1].y, h[2].x, h[2].y, Li, Lj, Vs);
+    double F[5];
+    compact_flux(F, un, h[1].y, h[2].x, h[2].y, Li, Lj, Vs);
     if (mf) {  // the closure's part of the face's mass flux
-      mf[(size_t(__ldg(m.erow + slice_)) + __ldg(m.qmap + q)) * 32 + (threadIdx.x & 31)] += dm;
+      mf[(size_t(__ldg(m.erow + slice_)) + __ldg(m.qmap + q)) * 32 + (threadIdx.x & 31)] -= F[0];
       q += 32 * parts_;
     }
+#pragma unroll
+    for (int c = 0; c < 5; ++c) acc[c] += F[c];
   }
   combine_parts(acc, smem, kSumBytes<double>(5), part_, parts_, t_ + spr_ < nsl_);
   if (valid && part_ == 0) {
@@ -765,7 +797,8 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad(CASE_ARGS) {
     ui[0] = a.x; ui[1] = a.y; ui[2] = c.x;
   }
   double g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 2
+  BlockSums<9, double> blocks(smem + 2 * pl, kSumBytes<double>(9));
+#pragma unroll 1
   while (rows.left > 0) {
     double c[3];
     const int jl = rows.next(parts_, c);
@@ -778,7 +811,9 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad(CASE_ARGS) {
       g[3 * d + 1] += cy * du[d];
       g[3 * d + 2] += cz * du[d];
     }
+    if (rows.left % kGradBlock == 0 && rows.left > 0) blocks.put(g);
   }
+  blocks.add_to(g);
   combine_parts(g, smem + 2 * pl, kSumBytes<double>(9), part_, parts_, t_ + spr_ < nsl_);
   if (valid && part_ == 0) {
     double* P = reinterpret_cast<double*>(s.V + i);
@@ -2313,7 +2348,7 @@ __global__ void k_expand_entries(long long E, long long Q, const int* __restrict
     if (f != kNoFace)
       for (int d = 0; d < 3; ++d) {
         v[d] = sg * n_ef[a + d];
-        v[3 + d] = 0.5 * c_ef[a + d];  // FlowSolver.hpp:2256-2259
+        v[3 + d] = c_ef[a + d];
       }
     double2* o = en + (k / 32) * 96 + (k & 31);
     for (int c = 0; c < 3; ++c) o[32 * c] = make_double2(v[2 * c], v[2 * c + 1]);
@@ -2344,12 +2379,13 @@ __global__ void k_fill_nbr(MeshDev m, int* __restrict__ nbr) {
   }
 }
 
-// FP32 copies of the entry geometry and gradient coefficients (mixed form)
+// FP32 copies of the entry geometry (with the c vectors halved, as
+// FlowSolver.hpp:2256-2259 keeps them) and gradient coefficients (mixed form)
 __global__ void k_geom32(long long ne, long long nq, long long nc, const double* __restrict__ en,
                          const double* __restrict__ qg, const double* __restrict__ gc, float* en32, float* qg32,
                          float* gc32) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t < ne) en32[t] = float(en[t]);
+  if (t < ne) en32[t] = float((t / 64 % 3 * 2 + (t & 1) >= 3) ? 0.5 * en[t] : en[t]);
   if (t < nq) qg32[t] = float(qg[t]);
   if (t < nc) gc32[t] = float(gc[t]);
 }
@@ -4079,6 +4115,7 @@ extern "C" int cgx_solver_create(cgx_mesh* m, const cgx_params* p, cgx_precision
   ph.h_ref = ph.R * p->gamma / (p->gamma - 1.0) * p->T_ref;
   ph.limit_asgs = p->limit_asgs;
   ph.invgm1 = 1.0 / (p->gamma - 1.0);
+  ph.gogm1 = p->gamma * ph.invgm1;
   const size_t N = m->N;
   s->nblocks = int((N + kBlock - 1) / kBlock);
   s->nitems = m->md.nitems;

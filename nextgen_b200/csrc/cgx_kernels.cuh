@@ -24,7 +24,8 @@
 //   erow[s+1]); a cell has cnt[i].x of them, and inside an item cells are
 //   ordered by that count, so that few lanes of a row are empty.
 //     extended faces: lidx[row][32] local index, en[row][3][32][2] {normal along
-//       the entry (negated for the face's second cell), the halved c vector}
+//       the entry (negated for the face's second cell), the c vector (halved in
+//       the FP32 copy)}
 //     compact faces (rows qrow, count cnt.y): clidx, qmap[row][32] (the cell's
 //       extended row of the same face), qg[row][3][32][2] {unit normal along
 //       the entry, area, area_over_delta, area/area_over_delta}
@@ -115,6 +116,7 @@ struct Phys {
   int diss_mode;
   int dt_mode;
   double dt_max;  // CFL_DT
+  double gogm1;   // gamma/(gamma-1)
   double h_ref;   // R gamma/(gamma-1) T_ref (mixed-precision offsets)
   int limit_asgs; // LIMIT_ASGS
   double invgm1;  // 1/(gamma-1)
@@ -181,7 +183,7 @@ struct MeshDev {
   const unsigned short* clidx;  // [qrow][32] neighbour in the item's compact union
   const unsigned short* qmap;   // [qrow][32] the entry's row among the cell's extended rows
   const unsigned short* cglidx; // [grow][32] neighbour in the item's compact union
-  const double* en;             // [erow][3][32][2] n (along the entry), c/2
+  const double* en;             // [erow][3][32][2] n (along the entry), c
   const double* qg;             // [qrow][3][32][2] unit normal, area, aod, delta
   const double* gc;             // [grow][3][32] gradient coefficients
   const double* vol;

@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad_f(CASE_ARGS) {
     ui[0] = a.x; ui[1] = a.y; ui[2] = a.z;
   }
   float g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 2
+  BlockSums<9, float> blocks(smem + pl, kSumBytes<float>(9));
+#pragma unroll 1
   while (rows.left > 0) {
     float c[3];
     const int jl = rows.next(parts_, c);
@@ -290,7 +291,9 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad_f(CASE_ARGS) {
       g[3 * d + 1] += cy * du[d];
       g[3 * d + 2] += cz * du[d];
     }
+    if (rows.left % kGradBlock == 0 && rows.left > 0) blocks.put(g);
   }
+  blocks.add_to(g);
   combine_parts(g, smem + pl, kSumBytes<float>(9), part_, parts_, t_ + spr_ < nsl_);
   if (valid && part_ == 0) {
     float* P = reinterpret_cast<float*>(s.VF + i);
