@@ -275,7 +275,10 @@ __device__ __forceinline__ double4 smem_Q(const int4* sm, int pl, int j) {
 // F holds M and twice the others, on the sums s = u_a + u_b = 2 uf and r =
 // 1/(v_a + v_b) = rho_f/2, so that no halves are left (powers of two: the same
 // roundings); qr = rho_a/4.  Every term changes sign exactly under (a <-> b,
-// n -> -n, c kept), so the two cells of a face see exactly opposite fluxes.
+// n -> -n, c kept), so the two cells of a face see exactly opposite fluxes: for
+// that, a cell's enthalpy is rounded to the same value (enthalpy()) whichever
+// side of the face it is on.
+__device__ __forceinline__ double enthalpy(double K, double p, double v) { return __dmul_rn(K, __dmul_rn(p, v)); }
 __device__ __forceinline__ void ext_flux(double F[5], const double n[3], const double c[3], const ERec& a, double qr,
                                          double ha, const ERec& b, double K) {
   const double r = rcp_nr(a.v + b.v);
@@ -292,7 +295,7 @@ __device__ __forceinline__ void ext_flux(double F[5], const double n[3], const d
   const double sdu = fma(s[2], du[2], fma(s[1], du[1], s[0] * du[0]));
   const double M = fma(r, w, sc * fma(0.25, b.rho, -qr));
   const double mc = sc * r;  // 2 mdot_c
-  const double hb = K * (b.p * b.v);
+  const double hb = enthalpy(K, b.p, b.v);
   const double ps = a.p + b.p, dp = b.p - a.p;
   F[0] = M;
 #pragma unroll
@@ -349,7 +352,7 @@ __device__ __forceinline__ void compact_flux(double F[5], const double un_[3], d
 #pragma unroll
   for (int d = 0; d < 3; ++d) F[1 + d] = fma(mu_aod, du[d], fma(mu_area, gn[d], fma(kn, un_[d], m * uf[d])));
   const double hs = fmax(vs.symh * rho_m * aun * half_aod - k_aod, 0.0);
-  const double pva = a.p * a.sp_vol, pvb = b.p * b.sp_vol;
+  const double pva = __dmul_rn(a.p, a.sp_vol), pvb = __dmul_rn(b.p, b.sp_vol);  // (not fused into one side's difference)
   const double de = dh - (pvb - pva);
   const double ufgn = uf[0] * gn[0] + uf[1] * gn[1] + uf[2] * gn[2];
   double e = mu_aod * (ufdu + un_m * dun * (1.0 / 3.0));
@@ -509,7 +512,8 @@ struct BlockSums {
 //   k_rhs_comp: rhs[i] -= sum over i's compact faces of the viscous/dissipation
 //               closure
 // Every face is evaluated by each of its two cells with the orientation
-// reversed (n -> -n, unit_n -> -unit_n, c kept), which gives the negated flux.
+// reversed (n -> -n, unit_n -> -unit_n, c kept), which gives the negated flux
+// (in FP64 bit for bit).
 //
 // k_rhs_ext streams 50 B per directed entry (about 80 a cell) and is bound by
 // HBM: 128^3 jittered cells 1.47 ms, 5.9 TB/s of rows (with an entry's six values
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   double hi = 0.0, qr = 0.0;
   if (valid) {
     smem_E(sE, pl, loc_, Ei);
-    hi = K * (Ei.p * Ei.v);
+    hi = enthalpy(K, Ei.p, Ei.v);
     qr = 0.25 * Ei.rho;
   }
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
