@@ -84,11 +84,15 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return fma(r, e, r);
 }
 
-// 256-bit read-only global loads (sm_100): a 32 B-aligned record piece per
-// lane in one instruction, one sector per lane.
+// 256-bit global loads (sm_100): a 32 B-aligned record piece per lane in one
+// instruction, one sector per lane.  Ordered after after_previous(): the records
+// are another kernel's stores.
 __device__ __forceinline__ double4 ld4(const void* p) {
   double4 r;
-  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+               : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w)
+               : "l"(p)
+               : "memory");
   return r;
 }
 __device__ __forceinline__ void st4(void* p, double a, double b, double c, double d) {
@@ -96,14 +100,13 @@ __device__ __forceinline__ void st4(void* p, double a, double b, double c, doubl
 }
 
 
-// dudx of one cell (g[8] with the last sector: symh, symp, mu_lam)
-__device__ __forceinline__ double4 load_Vg(const VRec* base, int j, double g[9]) {
+// dudx of one cell
+__device__ __forceinline__ void load_Vg(const VRec* base, int j, double g[9]) {
   const double* p = reinterpret_cast<const double*>(base + j);
   const double4 b = ld4(p + 4), c = ld4(p + 8), d = ld4(p + 12);
   g[0] = b.x; g[1] = b.y; g[2] = b.z; g[3] = b.w;
   g[4] = c.x; g[5] = c.y; g[6] = c.z; g[7] = c.w;
   g[8] = d.x;
-  return d;
 }
 
 // ---- shared-memory staging of neighbour records -------------------------
@@ -137,8 +140,11 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
 // Until after_previous() returns, i.e. until that kernel and with it all
 // earlier work is complete and visible, they touch only what no kernel of a
 // step writes: the mesh and the work list (their first rows are on their way
-// into L2 meanwhile).  Every CTA with work calls it.  launch_next() lets the
-// next kernel start.  One FP64 step of 8^3 cells 0.076 -> 0.064 ms, 48^3 0.604 ->
+// into L2 meanwhile).  Every CTA with work calls it.  What a kernel of a step
+// writes (the state and the packed records) is never read through __ldg or a
+// .nc load, before or after it: such loads need data that is read-only for as
+// long as the kernel runs, and are not kept behind this wait.  launch_next() lets
+// the next kernel start.  One FP64 step of 8^3 cells 0.076 -> 0.064 ms, 48^3 0.604 ->
 // 0.595, a batch of 12 boxes 1.5 % faster; nothing at 128^3.
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

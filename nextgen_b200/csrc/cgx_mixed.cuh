@@ -314,7 +314,7 @@ __device__ __forceinline__ int cell_props_f(const Phys& ph, const MeshDev& m, co
   {
     const float* vg = s.VF[i].g;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) g[c] = __ldg(vg + c);
+    for (int c = 0; c < 9; ++c) g[c] = vg[c];
   }
   const double2 cc01 = __ldg(reinterpret_cast<const double2*>(m.cc + i));
   const double2 cc23 = __ldg(reinterpret_cast<const double2*>(m.cc + i) + 1);
