@@ -2530,6 +2530,10 @@ int dupload(T** p, const std::vector<T, A>& v, size_t* acc, cgx_staging::Staging
 struct cgx_mesh {
   int device = 0;
   int N = 0, ncv_g2 = 0;
+  // Guards what solvers add to the mesh when the first of them needs it: the
+  // FP32 copies and the neighbour list in md, have32, allocs, bytes and stats.
+  // The rest is constant once the mesh is made.
+  mutable std::mutex mu;
   long long nq = 0, nc = 0;  // compact and gradient entries, empty lanes included
   bool have32 = false;
   std::vector<int> perm;  // new -> old
@@ -4077,6 +4081,7 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
 
 extern "C" int cgx_mesh_stats_get(const cgx_mesh* m, cgx_mesh_stats* out) {
   if (!m || !out) return fail(CGX_E_ARG, "null argument");
+  std::lock_guard<std::mutex> lk(m->mu);
   *out = m->stats;
   return CGX_OK;
 }
@@ -4156,6 +4161,7 @@ extern "C" int cgx_solver_create(cgx_mesh* m, const cgx_params* p, cgx_precision
     AL(sd.LF, N);
     AL(sd.VF, N);
     AL(sd.QF, N);
+    std::lock_guard<std::mutex> lk(m->mu);
     if (!m->have32) {
       float *en32, *qg32, *gc32;
       size_t* mb = &m->bytes;
@@ -4227,7 +4233,10 @@ extern "C" int cgx_solver_create(cgx_mesh* m, const cgx_params* p, cgx_precision
   {  // work list (the mesh's items) and the one-entry case table
     const std::vector<Item>& items = m->items;
     CaseDev cd{};
-    cd.m = m->md;
+    {
+      std::lock_guard<std::mutex> lk(m->mu);
+      cd.m = m->md;
+    }
     cd.s = sd;
     cd.ph = ph;
     cd.nitems = s->nitems;
@@ -4403,18 +4412,19 @@ extern "C" int cgx_get_state(cgx_solver* s, double* rho, double* u, double* rhoE
 
 // The extended entries' global neighbours, which only the scalars read, are
 // built when a solver of the mesh first has scalars (4 B per entry).
-static int ensure_nbr(cgx_mesh* m, cudaStream_t stream) {
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lk(mu);
-  if (m->md.nbr) return CGX_OK;
-  int* nbr = nullptr;
-  if (int rc = dalloc(&nbr, size_t(std::max(m->md.E, 1LL)), &m->bytes)) return rc;
-  m->allocs.push_back(nbr);
-  k_fill_nbr<<<m->md.nitems, 128, 0, stream>>>(m->md, nbr);
-  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
-    return fail(CGX_E_CUDA, "neighbour list of the scalars failed");
-  m->md.nbr = nbr;
-  m->stats.device_bytes = m->bytes;
+static int ensure_nbr(cgx_mesh* m, cudaStream_t stream, const int** out) {
+  std::lock_guard<std::mutex> lk(m->mu);
+  if (!m->md.nbr) {
+    int* nbr = nullptr;
+    if (int rc = dalloc(&nbr, size_t(std::max(m->md.E, 1LL)), &m->bytes)) return rc;
+    m->allocs.push_back(nbr);
+    k_fill_nbr<<<m->md.nitems, 128, 0, stream>>>(m->md, nbr);
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
+      return fail(CGX_E_CUDA, "neighbour list of the scalars failed");
+    m->md.nbr = nbr;
+    m->stats.device_bytes = m->bytes;
+  }
+  *out = m->md.nbr;
   return CGX_OK;
 }
 
@@ -4446,8 +4456,8 @@ extern "C" int cgx_set_scalars(cgx_solver* s, int nsc, const double* sc) {
     if (nsc > 0) {
       const size_t E = size_t(std::max(s->mesh->md.E, 1LL));
       int rc;
-      if ((rc = ensure_nbr(s->mesh, s->stream))) return rc;
-      s->hcase.m.nbr = s->run.dcase.m.nbr = s->mesh->md.nbr;
+      if ((rc = ensure_nbr(s->mesh, s->stream, &s->hcase.m.nbr))) return rc;
+      s->run.dcase.m.nbr = s->hcase.m.nbr;
       if ((rc = dalloc(&sd.sc, size_t(nsc) * N, &s->bytes))) return rc;
       s->allocs.push_back(sd.sc);
       if ((rc = dalloc(&sd.rhs_sc, 3 * size_t(nsc) * N, &s->bytes))) return rc;
@@ -5111,7 +5121,7 @@ extern "C" int cgx_calc_cfl(cgx_solver* s, double dt, double* cfl_max, double* c
   if (!s->inited) return fail(CGX_E_STATE, "cgx_init_complete not called");
   CK(cudaSetDevice(s->mesh->device));
   const int N = s->mesh->N;
-  k_cfl_cells<<<(N + kBlock - 1) / kBlock, kBlock, 0, s->stream>>>(s->mesh->md, s->sd, s->mesh->d_perm, dt, s->d_stage);
+  k_cfl_cells<<<(N + kBlock - 1) / kBlock, kBlock, 0, s->stream>>>(s->run.dcase.m, s->sd, s->mesh->d_perm, dt, s->d_stage);
   int rc = launch_check(s->run, 1);
   if (rc) return rc;
   std::vector<double> h(N);
@@ -5426,7 +5436,7 @@ extern "C" int cgx_totals(cgx_solver* s, double out[5]) {
   if (!s || !out) return fail(CGX_E_ARG, "null argument");
   CK(cudaSetDevice(s->mesh->device));
   const int nb = s->nblocks;
-  k_totals_partial<<<nb, kBlock, 0, s->stream>>>(s->mesh->md, s->sd, s->d_part);
+  k_totals_partial<<<nb, kBlock, 0, s->stream>>>(s->run.dcase.m, s->sd, s->d_part);
   k_totals_final<<<1, 32, 0, s->stream>>>(s->d_part, nb, s->d_part + 5 * size_t(nb));
   int rc = launch_check(s->run, 2);
   if (rc) return rc;
@@ -5559,7 +5569,11 @@ struct cgx_batch {
   std::vector<BatchCase> slots;  // slot index = position in the case table
   std::map<int, int> slot_of;    // case id -> slot
   int next_id = 0;
-  std::map<cgx_mesh*, int> mesh_refs;
+  struct MeshUse {
+    int cases = 0;
+    size_t bytes = 0;  // of the mesh when its first case joined: what `used` holds for it
+  };
+  std::map<cgx_mesh*, MeshUse> mesh_refs;
   CaseDev* d_cases = nullptr;
   Item* d_items = nullptr;
   int item_cap = 0;
@@ -5776,12 +5790,17 @@ extern "C" int cgx_batch_admit(cgx_batch* b, cgx_batch_case* pc, int* case_id) {
   if (slot < 0) return fail(CGX_E_OOM, "cgx_batch_admit: all case slots in use");
   cgx_mesh* mesh = pc->mesh;
   cgx_solver* s = pc->s;
-  const size_t need = s->bytes + (b->mesh_refs.count(mesh) ? 0 : mesh->bytes);
+  size_t mesh_bytes = 0;
+  {
+    std::lock_guard<std::mutex> lk(mesh->mu);
+    if (!b->mesh_refs.count(mesh)) mesh_bytes = mesh->bytes;
+    s->hcase.m = mesh->md;  // mesh records as of now
+  }
+  const size_t need = s->bytes + mesh_bytes;
   if (b->used + need > b->budget) return fail(CGX_E_OOM, "cgx_batch_admit: HBM budget exceeded");
   CK(cudaSetDevice(b->device));
-  // the case's descriptor into the table (mesh records as of now), ordered
-  // before the next step on the batch's stream
-  s->hcase.m = mesh->md;
+  // the case's descriptor into the table, ordered before the next step on the
+  // batch's stream
   CK(cudaMemcpyAsync(b->d_cases + slot, &s->hcase, sizeof(CaseDev), cudaMemcpyHostToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   BatchCase& c = b->slots[slot];
@@ -5793,7 +5812,8 @@ extern "C" int cgx_batch_admit(cgx_batch* b, cgx_batch_case* pc, int* case_id) {
   c.finished = (pc->target == 0);
   c.bytes = s->bytes;
   b->used += need;
-  b->mesh_refs[mesh]++;
+  cgx_batch::MeshUse& use = b->mesh_refs[mesh];
+  if (use.cases++ == 0) use.bytes = mesh_bytes;
   b->slot_of[c.id] = slot;
   b->dirty = true;
   delete pc;
@@ -5812,8 +5832,11 @@ extern "C" int cgx_batch_add(cgx_batch* b, cgx_mesh* mesh, const cgx_params* p, 
   if (!free_slot) return fail(CGX_E_OOM, "cgx_batch_add: all case slots in use");
   // the footprint checked before anything is allocated
   size_t need = solver_bytes(mesh->N, mesh->md.nitems, b->prec);
-  if (!b->mesh_refs.count(mesh)) need += mesh->bytes;
-  if (b->prec == CGX_MIXED && !mesh->have32) need += mesh32_bytes(mesh);
+  {
+    std::lock_guard<std::mutex> lk(mesh->mu);
+    if (!b->mesh_refs.count(mesh)) need += mesh->bytes;
+    if (b->prec == CGX_MIXED && !mesh->have32) need += mesh32_bytes(mesh);
+  }
   if (b->used + need > b->budget) return fail(CGX_E_OOM, "cgx_batch_add: HBM budget exceeded");
   cgx_batch_case* pc = nullptr;
   int rc = cgx_batch_prepare(b, mesh, p, rho, u, pres, nsteps, &pc);
@@ -5935,8 +5958,9 @@ extern "C" int cgx_batch_remove(cgx_batch* b, int case_id) {
   CK(cudaStreamSynchronize(b->stream));
   BatchCase& c = b->slots[it->second];
   b->used -= c.bytes;
-  if (--b->mesh_refs[c.mesh] == 0) {
-    b->used -= c.mesh->bytes;
+  cgx_batch::MeshUse& use = b->mesh_refs[c.mesh];
+  if (--use.cases == 0) {
+    b->used -= use.bytes;
     b->mesh_refs.erase(c.mesh);
   }
   cgx_solver_destroy(c.s);
