@@ -4428,10 +4428,28 @@ static int ensure_nbr(cgx_mesh* m, cudaStream_t stream, const int** out) {
   return CGX_OK;
 }
 
+// a new source configuration or other scalar arrays change what the step graphs
+// hold
+static void drop_graphs(cgx_solver* s) {
+  for (cudaGraphExec_t* g : {&s->hgraph, &s->tgraph})
+    if (*g) {
+      cudaGraphExecDestroy(*g);
+      *g = nullptr;
+    }
+  if (s->pgraph) {
+    cudaGraphExecDestroy(s->pgraph);
+    s->pgraph = nullptr;
+  }
+  if (s->graph) {
+    cudaGraphExecDestroy(s->graph);
+    s->graph = nullptr;
+  }
+}
+
 // The scalar arrays (sc, three stages of rhs_sc, per-entry mf) are allocated
 // at the first call with nsc > 0 and kept; a later call with another nsc
 // reallocates them.  Every copy of the case descriptor (host, device table,
-// the runner's by-value copy) is refreshed and the step graph re-captured.
+// the runner's by-value copy) is refreshed and the step graphs re-captured.
 extern "C" int cgx_set_scalars(cgx_solver* s, int nsc, const double* sc) {
   if (!s) return fail(CGX_E_ARG, "cgx_set_scalars: null solver");
   if (nsc < 0 || nsc > kMaxScalars) return fail(CGX_E_ARG, "cgx_set_scalars: nsc out of range 0..8");
@@ -4470,14 +4488,7 @@ extern "C" int cgx_set_scalars(cgx_solver* s, int nsc, const double* sc) {
     s->hcase.s = sd;
     s->run.dcase.s = sd;
     CK(cudaMemcpyAsync(s->d_case, &s->hcase, sizeof(CaseDev), cudaMemcpyHostToDevice, s->stream));
-    if (s->pgraph) {
-      cudaGraphExecDestroy(s->pgraph);
-      s->pgraph = nullptr;
-    }
-    if (s->graph) {
-      cudaGraphExecDestroy(s->graph);
-      s->graph = nullptr;
-    }
+    drop_graphs(s);
   }
   if (nsc > 0) {
     if (size_t(nsc) * N > 9 * N) return fail(CGX_E_ARG, "cgx_set_scalars: staging too small");
@@ -4520,23 +4531,6 @@ extern "C" int cgx_get_rhs_sc(cgx_solver* s, int rk_stage, double* rhs_sc) {
   if ((rc = device_to_host(s, rhs_sc, s->d_stage, size_t(nsc) * N * sizeof(double)))) return rc;
   CK(cudaStreamSynchronize(s->stream));
   return CGX_OK;
-}
-
-// a new source configuration changes what the step graphs hold
-static void drop_graphs(cgx_solver* s) {
-  for (cudaGraphExec_t* g : {&s->hgraph, &s->tgraph})
-    if (*g) {
-      cudaGraphExecDestroy(*g);
-      *g = nullptr;
-    }
-  if (s->pgraph) {
-    cudaGraphExecDestroy(s->pgraph);
-    s->pgraph = nullptr;
-  }
-  if (s->graph) {
-    cudaGraphExecDestroy(s->graph);
-    s->graph = nullptr;
-  }
 }
 
 static int check_frame_velocities(const cgx_solver* s);
