@@ -2476,6 +2476,7 @@ int dalloc(T** p, size_t n, size_t* acc) {
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
   if (e != cudaSuccess) {
     g_err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    cudaGetLastError();  // reported here, not by a later launch's check
     return e == cudaErrorMemoryAllocation ? CGX_E_OOM : CGX_E_CUDA;
   }
   if (acc) *acc += bytes;
@@ -4471,24 +4472,38 @@ extern "C" int cgx_set_scalars(cgx_solver* s, int nsc, const double* sc) {
     }
     sd.sc = sd.rhs_sc = sd.mf = nullptr;
     sd.nsc = 0;
+    int rc = CGX_OK;
     if (nsc > 0) {
+      // all of the arrays or, where memory runs out, none: the solver then has no
+      // scalars
       const size_t E = size_t(std::max(s->mesh->md.E, 1LL));
-      int rc;
-      if ((rc = ensure_nbr(s->mesh, s->stream, &s->hcase.m.nbr))) return rc;
-      s->run.dcase.m.nbr = s->hcase.m.nbr;
-      if ((rc = dalloc(&sd.sc, size_t(nsc) * N, &s->bytes))) return rc;
-      s->allocs.push_back(sd.sc);
-      if ((rc = dalloc(&sd.rhs_sc, 3 * size_t(nsc) * N, &s->bytes))) return rc;
-      s->allocs.push_back(sd.rhs_sc);
-      if ((rc = dalloc(&sd.mf, E, &s->bytes))) return rc;
-      s->allocs.push_back(sd.mf);
-      CK(cudaMemsetAsync(sd.rhs_sc, 0, 3 * size_t(nsc) * N * sizeof(double), s->stream));
-      sd.nsc = nsc;
+      double *a_sc = nullptr, *a_rhs = nullptr, *a_mf = nullptr;
+      const size_t bytes = s->bytes;
+      if (!(rc = ensure_nbr(s->mesh, s->stream, &s->hcase.m.nbr)) &&
+          !(rc = dalloc(&a_sc, size_t(nsc) * N, &s->bytes)) &&
+          !(rc = dalloc(&a_rhs, 3 * size_t(nsc) * N, &s->bytes)) && !(rc = dalloc(&a_mf, E, &s->bytes)) &&
+          cudaMemsetAsync(a_rhs, 0, 3 * size_t(nsc) * N * sizeof(double), s->stream) != cudaSuccess)
+        rc = fail(CGX_E_CUDA, "cgx_set_scalars: clearing the rhs failed");
+      if (rc) {
+        for (double* q : {a_sc, a_rhs, a_mf}) cudaFree(q);
+        s->bytes = bytes;
+      } else {
+        s->run.dcase.m.nbr = s->hcase.m.nbr;
+        sd.sc = a_sc;
+        sd.rhs_sc = a_rhs;
+        sd.mf = a_mf;
+        sd.nsc = nsc;
+        for (double* q : {a_sc, a_rhs, a_mf}) s->allocs.push_back(q);
+      }
     }
     s->hcase.s = sd;
     s->run.dcase.s = sd;
-    CK(cudaMemcpyAsync(s->d_case, &s->hcase, sizeof(CaseDev), cudaMemcpyHostToDevice, s->stream));
     drop_graphs(s);
+    CK(cudaMemcpyAsync(s->d_case, &s->hcase, sizeof(CaseDev), cudaMemcpyHostToDevice, s->stream));
+    if (rc) {
+      cudaStreamSynchronize(s->stream);
+      return rc;
+    }
   }
   if (nsc > 0) {
     if (size_t(nsc) * N > 9 * N) return fail(CGX_E_ARG, "cgx_set_scalars: staging too small");
