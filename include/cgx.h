@@ -161,10 +161,10 @@ int cgx_solver_destroy(cgx_solver* s);
 /* Conserved state in reference order (host arrays).  Host arrays may be
  * page-locked (copied directly) or pageable, such as a host solver's new[]
  * arrays: pageable arrays of 4 MiB or more are staged through two pinned 64
- * MiB chunks (allocated at first use; at most two such pairs stay with the
- * process, for its later calls and meshes), which is several times faster than
- * a pageable copy.  The same holds for every call below that
- * takes or fills a host array of cells. */
+ * MiB chunks (allocated at first use and kept for later calls and meshes: as many
+ * such pairs as solvers of a device have needed at once, two when they are gone),
+ * which is several times faster than a pageable copy.  The same holds for every
+ * call below that takes or fills a host array of cells. */
 int cgx_set_state(cgx_solver* s, const double* rho, const double* u, const double* rhoE);
 /* rho, u, p; rhoE = p/(gamma-1) + 0.5 rho |u|^2 (IdealGasSolver.hpp:275-301). */
 int cgx_set_state_primitive(cgx_solver* s, const double* rho, const double* u,

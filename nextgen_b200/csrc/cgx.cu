@@ -2644,6 +2644,7 @@ struct cgx_solver {
   cudaEvent_t oev = nullptr;
   cudaEvent_t pev[9] = {};
   std::unique_ptr<cgx_staging::Staging> staging;  // for pageable caller arrays, during a call
+  std::unique_ptr<cgx_staging::User> staging_user;  // from the first of them on
   std::atomic<long long> launches{0};
   SourceCfg src;
   std::vector<BcZone> bc;   // boundary conditions per zone (host copy of sd.bc)
@@ -4317,6 +4318,7 @@ static bool page_locked(const void* p) {
 
 static int staging_of(cgx_solver* s, cgx_staging::Staging** st) {
   if (!s->staging) {
+    if (!s->staging_user) s->staging_user.reset(new cgx_staging::User(s->mesh->device));
     std::unique_ptr<cgx_staging::Staging> n(new cgx_staging::Staging(s->stream));
     const cudaError_t e = n->init();
     if (e != cudaSuccess)
