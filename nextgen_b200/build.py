@@ -63,7 +63,8 @@ def build_meshgen(force=False):
 def build_cgx(force=False, verbose=False):
     out = os.path.join(LIB, "libcgx.so")
     ops_obj = os.path.join(LIB, "cgx_ops.o")
-    srcs = [os.path.join(CSRC, f) for f in ("cgx.cu", "cgx_kernels.cuh", "cgx_mixed.cuh", "cgx_ops.cu", "svd33.h")] + \
+    srcs = [os.path.join(CSRC, f) for f in ("cgx.cu", "cgx_kernels.cuh", "cgx_mixed.cuh", "cgx_ops.cu", "host_staging.h",
+                                                "svd33.h")] + \
         [os.path.join(INC, h) for h in ("cgx.h", "cgx_ops.h", "cgx_meshgen.h")]
     if force or _stale(out, srcs):
         os.makedirs(LIB, exist_ok=True)
