@@ -3086,15 +3086,21 @@ int enqueue_step_end(const Runner& R, int mode) { return end_var(R, R.tune.g_end
 std::mutex g_tune_mu;
 std::map<int, Tune> g_tune_cache;
 
-int tune_bucket(long long ncells, cgx_precision prec) {
-  int b = 0;
+// What a choice of lane counts holds for: log2 of the cell count, that of the
+// mean item length (rounded up: a mesh's last item is short) and the precision,
+// in a single mesh or a batch.  The item length matters most: with 32-cell items
+// every lane count is one and the same launch, so a choice made there says
+// nothing about 128-cell items.
+int tune_bucket(long long ncells, long long nitems, bool direct, cgx_precision prec) {
+  const long long mean = nitems > 0 ? (ncells + nitems - 1) / nitems : 1;
+  int b = 0, l = 0;
   for (long long n = ncells; n > 1; n >>= 1) ++b;
-  return b * 4 + int(prec);
+  while ((1LL << l) < mean) ++l;
+  return ((b * 16 + l) * 2 + int(direct)) * 4 + int(prec);
 }
 
 // Time each candidate lane count of each kernel on the runner's cases and
-// keep the fastest; results are cached per size bucket (log2 of the cell
-// count) and precision.  All candidates compute the same values (only the
+// keep the fastest; results are cached per tune_bucket.  All candidates compute the same values (only the
 // order of the per-cell sums changes), and none changes the state.
 // CGX_TUNE="ext,comp,grad,end" (lanes per cell) skips the timing and fixes
 // the lane counts, e.g. to profile one variant.
@@ -3115,10 +3121,10 @@ bool fixed_tune(Tune* t) {
   return true;
 }
 
-int autotune(Runner& run, long long ncells) {
+int autotune(Runner& run, long long ncells, long long nitems) {
   Runner R = run;
   R.overlap = false;
-  const int bucket = tune_bucket(ncells, R.prec);
+  const int bucket = tune_bucket(ncells, nitems, R.direct, R.prec);
   if (fixed_tune(&run.tune)) return CGX_OK;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -5075,7 +5081,7 @@ static int init_complete(cgx_solver* s, bool tune) {
   if (rc) return rc;
   if ((rc = cgx_calc_sgs_props(s))) return rc;
   if (tune) {
-    if ((rc = autotune(s->run, s->mesh->N))) return rc;
+    if ((rc = autotune(s->run, s->mesh->N, s->nitems))) return rc;
     // recompute with the tuned lane counts so that the initial packed state,
     // gradient and properties do not depend on whether tuning ran or was cached
     if ((rc = cgx_update_primitive(s))) return rc;
@@ -5866,10 +5872,10 @@ extern "C" int cgx_batch_step(cgx_batch* b, int nsteps, int* n_done) {
     if (b->nitems == 0) break;
     // lane counts for this batch size (cached per bucket); re-derive the
     // gradients with the chosen counts afterwards
-    const int bucket = tune_bucket(b->active_cells, b->prec);
+    const int bucket = tune_bucket(b->active_cells, b->nitems, false, b->prec);
     if (bucket != b->tuned_bucket) {
       const Tune old = b->run.tune;
-      if ((rc = autotune(b->run, b->active_cells))) return rc;
+      if ((rc = autotune(b->run, b->active_cells, b->nitems))) return rc;
       const Tune& t = b->run.tune;
       if (b->tuned_bucket < 0 || t.g_ext != old.g_ext || t.g_comp != old.g_comp || t.g_grad != old.g_grad ||
           t.g_end != old.g_end) {
