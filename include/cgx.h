@@ -23,7 +23,7 @@
  *     calling thread.
  *   - Host arrays are in the caller's (reference) cell numbering and layout:
  *     rho[ncv], u[ncv][3], rhoE[ncv], rhs[ncv][5] = {rho, rhou[3], rhoE}.
- *     The library renumbers cells internally on a space-filling curve and
+ *     The library renumbers cells internally by recursive bisection and
  *     keeps the permutation.
  *   - The library owns all device memory.  A solver handle is not
  *     thread-safe; all of its work is ordered on one CUDA stream.
@@ -105,7 +105,7 @@ void cgx_params_default(cgx_params* p);
  * diagonal first) with cvocv_grad_coeff; extended faces cvoef/n_ef/c_ef with
  * c_ef NOT halved (as StaticSolver stores it); dcmag_hat_cv and
  * sa_to_vol_ratio as FlowSolver::init() computes them.  x_cv[ncv][3] is
- * optional: when given, cells are renumbered on a space-filling curve of x_cv.
+ * optional: when given, cells are renumbered by recursive bisection of x_cv.
  */
 typedef struct cgx_mesh_desc {
   int ncv, ncv_g2;

@@ -58,9 +58,8 @@ namespace {
 thread_local std::string g_err;
 
 constexpr int kBlock = 128;
-constexpr int kMaxRounds = 16;  // most rounds per item of a once-per-step kernel
 // largest neighbour unions an item may have (shared-memory budget of the
-// staged face kernels: 64 B per extended-face neighbour record, 192 B per
+// staged face kernels: 48 B per extended-face neighbour record, 192 B per
 // compact-face one)
 constexpr int kMaxUnionExt = 3000;
 constexpr int kMaxUnionComp = 1100;
@@ -2834,13 +2833,11 @@ void launch_grad(const Runner& R) {
 }
 template <int G, bool MIX>
 void launch_ext(const Runner& R, int st) {
-  if constexpr (G > 1)  // an item with a huge halo leaves room for few warps
-    if (smem_ext<G>(R) > size_t(g_smem_optin)) return launch_ext<1, MIX>(R, st);
   R.direct ? launch_ext_d<G, MIX, true>(R, st) : launch_ext_d<G, MIX, false>(R, st);
 }
 template <int G, bool MIX>
 void launch_comp(const Runner& R, int st) {
-  if constexpr (G > 1)  // an item with a huge halo leaves room for few warps
+  if constexpr (G > 8)  // 1100 records and the sums of 16 warps would be 227.2 KB
     if (smem_comp<G>(R) > size_t(g_smem_optin)) return launch_comp<1, MIX>(R, st);
   R.direct ? launch_comp_d<G, MIX, true>(R, st) : launch_comp_d<G, MIX, false>(R, st);
 }
@@ -3358,9 +3355,9 @@ extern "C" void cgx_params_default(cgx_params* p) {
 // cells: 16^3 0.077 / 0.098 / 0.138 ms, 24^3 0.122 / 0.147 / 0.160; with 64 /
 // 128: 32^3 0.287 / 0.265 FP64 and 0.179 / 0.226 mixed.  A batch of many small
 // boxes fills the GPU either way and loses 4 % with the short items.
-static int item_cells(int N) {
+static int item_cells(int N, int sms) {
   for (int c = kItemCells; c > kSlice; c /= 2)
-    if ((long long)N >= 2LL * 148 * c) return c;
+    if ((long long)N >= 2LL * sms * c) return c;
   return kSlice;
 }
 
@@ -3485,7 +3482,9 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
       if (d->icv_owner_g[g] < 0 || d->icv_owner_g[g] >= N) return bail(fail(CGX_E_ARG, "ghost owner out of range"));
     auto owner = [&](int idx) { return idx < N ? idx : d->icv_owner_g[idx - N]; };
     // ---- renumbering: each work item's cells are a compact block of x_cv
-    const int icells = item_cells(N);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int icells = item_cells(N, sms);
     std::vector<int>& perm = M->perm;
     perm.resize(N);
     std::iota(perm.begin(), perm.end(), 0);
@@ -3868,7 +3867,7 @@ extern "C" int cgx_mesh_create(const cgx_mesh_desc* d, int device, cgx_mesh** ou
     }
     PT.mark("items and halos");
     // ---- rows of the slices: counts, row offsets, then each slice's entries
-    // placed row by row in the order that place_entries chooses
+    // placed row by row in the order that RowOrder::place chooses
     const int nslice = (N + kSlice - 1) / kSlice;
     std::vector<ushort4> cnt(N);
     std::vector<int> erow(nslice + 1, 0), qrow(nslice + 1, 0), grow(nslice + 1, 0);
@@ -4200,7 +4199,7 @@ extern "C" int cgx_solver_create(cgx_mesh* m, const cgx_params* p, cgx_precision
     AL(sd.Q, N);
   }
   AL(sd.ctl, 1);
-  AL(sd.red, 2 * size_t(s->nitems) * kMaxRounds);
+  AL(sd.red, 2 * size_t(s->nitems));
   AL(s->d_case, 1);
   AL(s->d_items, s->nitems);
   AL(s->d_nitems, 1);
@@ -4258,7 +4257,6 @@ extern "C" int cgx_solver_create(cgx_mesh* m, const cgx_params* p, cgx_precision
     R.cases = s->d_case;
     R.items = s->d_items;
     R.nitems = s->d_nitems;
-    R.grid = s->nitems * kMaxRounds;
     R.nitems_host = s->nitems;
     R.direct = true;
     R.dcase = cd;
@@ -5556,7 +5554,7 @@ size_t solver_bytes(long long N, long long nitems, cgx_precision prec) {
   size_t rec = (prec == CGX_MIXED) ? sizeof(LRecF) + sizeof(VRecF) + sizeof(QRecF)
                                    : sizeof(LRec) + sizeof(VRec) + sizeof(QRec);
   return size_t(N) * (5 + 15 + 9 + 10) * sizeof(double) + size_t(N) * rec + sizeof(Ctl) +
-         size_t(2 * nitems) * kMaxRounds * sizeof(double) + sizeof(CaseDev) + size_t(nitems) * sizeof(Item) +
+         size_t(2 * nitems) * sizeof(double) + sizeof(CaseDev) + size_t(nitems) * sizeof(Item) +
          sizeof(int) + size_t(5 * nblocks + 5) * sizeof(double) + 4096;
 }
 

@@ -1,7 +1,7 @@
 // cgx_kernels.cuh -- device-side records of the B200 compressible-LES
 // right-hand side.
 //
-// Data layout in HBM (cells renumbered on a space-filling curve, "new" order):
+// Data layout in HBM (cells renumbered by recursive bisection, "new" order):
 //   state    rho[N], u0[N], u1[N], u2[N], rhoE[N]          (SoA, FP64)
 //   rhs      rhs[stage][5][N]                              (SoA, FP64)
 //   LRec[N]  {u0,u1,u2, 1/rho, p, rho, h, sos}  64 B       neighbour gathers

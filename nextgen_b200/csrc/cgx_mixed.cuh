@@ -25,7 +25,7 @@ struct FluxF {
   float rho, ru[3], rE;
 };
 
-// FP32 records in the swizzled shared arrays
+// FP32 records in shared memory
 __device__ __forceinline__ void smem_LF(const int4* sm, int pl, int j, LRecF& r) {
   const float4* p = reinterpret_cast<const float4*>(sm) + j;
   const float4 a = p[0], b = p[pl];
