@@ -1,7 +1,7 @@
-"""Every lane-count variant the autotuner can choose gives calcRhs within
-the face-sum tolerance of the oracle, so the variant picked on any mesh is
-a correct one.  Lane counts per kernel are forced through CGX_TUNE
-(extended faces, compact closures, gradient, once-per-step)."""
+"""Lane-count variants on a small box, whose items are single slices of 32 cells,
+give calcRhs within the face-sum tolerance of the oracle (the variants on items of
+several slices: test_gpu_row_edges.py).  Lane counts per kernel are forced through
+CGX_TUNE (extended faces, compact closures, gradient, once-per-step)."""
 import os
 
 import numpy as np
