@@ -521,7 +521,8 @@ struct BlockSums {
 // (in FP64 bit for bit).
 //
 // k_rhs_ext streams 50 B per directed entry (about 80 a cell) and is bound by
-// HBM: 128^3 jittered cells 1.47 ms, 5.9 TB/s of rows (with an entry's six values
+// HBM: 128^3 jittered cells 1.46 ms, 200^3 5.66 ms, i.e. 0.97 of a copy's rate by
+// its 4490 DRAM bytes a cell (with an entry's six values
 // in planes of their own and G neighbouring lanes per cell, whose sums 40
 // shuffles a cell combined, 1.73 ms; 200^3 7.95 ms, where each CTA's seven
 // streams also missed the TLB).  A ring of rows in shared memory, filled by
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
 }
 
 // 12 chunks of 16 bytes come from shared memory per entry besides its 50 B row,
-// and about 110 FP64 instructions follow: 128^3 0.88 ms (1.02 with G
+// and about 110 FP64 instructions follow: 128^3 0.87 to 0.91 ms (1.02 with G
 // neighbouring lanes per cell), 16 warps an SM at 128 registers.
 template <int G, bool DIRECT>
 __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 3 : G <= 8 ? 2 : 1) k_rhs_comp(CASE_ARGS, int stage) {
@@ -787,7 +788,7 @@ __global__ void __launch_bounds__(kItemCells) k_rk_prim(CASE_ARGS, int nw, doubl
 // _calcCvGradRange over the compact stencil (the reference's cvocv); the
 // velocities of the item's compact-face union are staged in shared memory (the
 // first 32 bytes of each LRec) and read through the entries' local indices.
-// 128^3: 0.266 ms (0.345 with G neighbouring lanes per cell).
+// 128^3: 0.270 ms (0.345 with G neighbouring lanes per cell).
 template <int G, bool DIRECT>
 __global__ void __launch_bounds__(kThreads<G>()) k_grad(CASE_ARGS) {
   extern __shared__ int4 smem[];
@@ -1011,7 +1012,7 @@ __device__ __forceinline__ void item_partial(double cmax, int anynan, const Stat
 // extended-face union of QRec and the CFL sum its compact-face union of LRec,
 // both staged in shared memory; the properties (logarithm, exponentials, square
 // roots in FP64) are then evaluated with every lane of part 0 on a cell of its
-// own.  128^3: 0.985 ms (1.17 with G neighbouring lanes per cell, one of which
+// own.  128^3: 0.975 ms (1.17 with G neighbouring lanes per cell, one of which
 // evaluated the properties).  Faces and properties in two kernels, the latter
 // with a thread per cell at 24 warps an SM, took 1.05.
 // mode bit 0: advance time/step by the dt just used; bit 1: set dt from CFL.
