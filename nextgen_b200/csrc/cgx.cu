@@ -143,8 +143,13 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
 // writes (the state and the packed records) is never read through __ldg or a
 // .nc load, before or after it: such loads need data that is read-only for as
 // long as the kernel runs, and are not kept behind this wait.  launch_next() lets
-// the next kernel start.  One FP64 step of 8^3 cells 0.076 -> 0.064 ms, 48^3 0.604 ->
-// 0.595, a batch of 12 boxes 1.5 % faster; nothing at 128^3.
+// the next kernel start: a staged kernel calls it when its records are staged.
+// At its start, the next kernel's CTAs fill up what a grid that fits at once leaves
+// free, unevenly over the SMs, and wait there in the way; at its end, less is
+// hidden.  Steps of jittered boxes with lane counts 4, 2, 2, 2, without overlap / at
+// the start / when staged / at the end: 16^3 FP64 0.084 / 0.086 / 0.070 / 0.074 ms,
+// mixed 0.074 / 0.065 / 0.061 / 0.066, 45^3 FP64 0.577 / 0.556 / 0.556 / 0.570; with
+// 1, 1, 1, 1 24^3 mixed 0.104 / 0.112 / 0.090 / 0.097.
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -405,7 +410,6 @@ __host__ __device__ constexpr int kSumBytes(int NV) {
 // DIRECT (a template parameter of every step kernel): one case passed by value
 // in `dcase`, items read from its mesh's own item table.
 #define STAGED_LOOP_BEGIN(G)                                                   \
-  launch_next();                                                               \
   const int n_items_ = DIRECT ? dcase.nitems : *nitems;                        \
   for (int v_ = blockIdx.x; v_ < n_items_; v_ += gridDim.x) {                  \
     const Item it_ = DIRECT ? dcase.m.items[v_] : items[v_];                   \
@@ -541,6 +545,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   stage_records<kEChunks, 4>(sE, pl, s.L, it_, m.hcell + it_.hoff, it_.nh);
   const double K = CASE_PH.gogm1;
   stage_wait();
+  launch_next();
   SLICES_BEGIN(G)
   ERec Ei;
   double hi = 0.0, qr = 0.0;
@@ -594,6 +599,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 3 : G <= 8 ? 2 : 1) k_
   stage_records<4, 4>(sL, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_records<8, 8>(sV, pv, s.V, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
+  launch_next();
   SLICES_BEGIN(G)
   LRec Li;
   if (valid) smem_L(sL, pl, loc_, Li);
@@ -799,6 +805,7 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad(CASE_ARGS) {
   after_previous();
   stage_records<2, 4>(smem, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
+  launch_next();
   const double2* su = reinterpret_cast<const double2*>(smem);
   SLICES_BEGIN(G)
   double ui[3] = {0.0, 0.0, 0.0};
@@ -1034,6 +1041,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 5 : G <= 8 ? 3 : 1) k_
   stage_records<2, 2>(sQ, pq, s.Q, it_, m.hcell + it_.hoff, it_.nh);
   stage_records<4, 4>(sL, pl, s.L, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
+  launch_next();
   // limitAsgs's dt: this step's, or outside a step the control block's
   const double dt_sgs = (mode & 1) ? s.ctl->dt : s.ctl->dt_sgs;
   double cmax = 0.0;

@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 8 : G <= 8 ? 4 : 1) k_
   stage_records<2, 2>(sL, pl, s.LF, it_, m.hcell + it_.hoff, it_.nh);
   const double h_ref = CASE_PH.h_ref;
   stage_wait();
+  launch_next();
   SLICES_BEGIN(G)
   LRecF Li;
   if (valid) smem_LF(sL, pl, loc_, Li);
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   const double h_ref = CASE_PH.h_ref;
   const float p_ref = float(CASE_PH.p_ref);
   stage_wait();
+  launch_next();
   SLICES_BEGIN(G)
   LRecF Li;
   if (valid) smem_LF(sL, pl, loc_, Li);
@@ -269,6 +271,7 @@ __global__ void __launch_bounds__(kThreads<G>()) k_grad_f(CASE_ARGS) {
   after_previous();
   stage_records<1, 2>(smem, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
+  launch_next();
   const float4* su = reinterpret_cast<const float4*>(smem);
   SLICES_BEGIN(G)
   float ui[3] = {0.0f, 0.0f, 0.0f};
@@ -397,6 +400,7 @@ __global__ void __launch_bounds__(kThreads<G>(), G == 1 ? 6 : G <= 8 ? 3 : 1) k_
   stage_records<1, 1>(sQ, pq, s.QF, it_, m.hcell + it_.hoff, it_.nh);
   stage_records<2, 2>(sL, pl, s.LF, it_, m.chcell + it_.choff, it_.nch);
   stage_wait();
+  launch_next();
   // limitAsgs's dt: this step's, or outside a step the control block's
   const double dt_sgs = (mode & 1) ? s.ctl->dt : s.ctl->dt_sgs;
   double cmax = 0.0;
