@@ -525,8 +525,8 @@ struct BlockSums {
 // (in FP64 bit for bit).
 //
 // k_rhs_ext streams 50 B per directed entry (about 80 a cell) and is bound by
-// HBM: 128^3 jittered cells 1.46 ms, 200^3 5.66 ms, i.e. 0.97 of a copy's rate by
-// its 4490 DRAM bytes a cell (with an entry's six values
+// HBM: 128^3 jittered cells 1.46 ms, 200^3 5.66 to 5.98 ms with the clock, i.e.
+// 0.97 to 0.92 of a copy's rate by its 4490 DRAM bytes a cell (with an entry's six values
 // in planes of their own and G neighbouring lanes per cell, whose sums 40
 // shuffles a cell combined, 1.73 ms; 200^3 7.95 ms, where each CTA's seven
 // streams also missed the TLB).  A ring of rows in shared memory, filled by
